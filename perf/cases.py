@@ -274,6 +274,118 @@ def run(state):
     return out + state["weights"]
 
 
+# ---------------------------------------------------------------------------- the same results in 64 bits
+#: step triples of the iteration (Polar Express, arXiv 2505.16932, with a safety factor of 1.05)
+_TRIPLES = [(a / 1.05, b / 1.05**3, c / 1.05**5) for a, b, c in (
+    (8.28721201814563, -23.595886519098837, 17.300387312530933),
+    (4.107059111542203, -2.9478499167379106, 0.5448431082926601),
+    (3.9486908534822946, -2.908902115962949, 0.5518191394370137),
+    (3.3184196573706015, -2.488488024314874, 0.51004894012372),
+    (2.300652019954817, -1.6689039845747493, 0.4188073119525673))]
+
+
+def _exact_newton_schulz(g):
+    x = g.double()
+    tall = x.shape[0] > x.shape[1]
+    x = x.T if tall else x
+    x = x / (x.norm() + 1e-7)
+    for a, b, c in _TRIPLES:
+        r = x @ x.T
+        x = a * x + (b * r + c * (r @ r)) @ x
+    return x.T if tall else x
+
+
+def _exact_muon(weight, grad):
+    """First step: momentum 0.95 with Nesterov, decoupled decay 0.1, update RMS 0.2."""
+    step = _exact_newton_schulz(1.95 * grad) * (_LR * 0.2 * math.sqrt(max(grad.shape)))
+    return weight.double() * (1 - _LR * 0.1) - step
+
+
+def _exact_adamw(weight, grad):
+    """First step: the bias-corrected averages are the gradient and its square; decay 0.01."""
+    return weight * (1 - _LR * 0.01) - _LR * grad / (grad.abs() + 1e-8)
+
+
+def _exact_decoder(cfg, p, ids):
+    """The decoder on a dictionary of parameters: pre-RMSNorm, rotate-half positions, grouped-query attention, SwiGLU."""
+    def norm(x, w):
+        return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + cfg.norm_eps) * w
+
+    b, s = ids.shape
+    d, kv = cfg.head_dim, cfg.n_kv_heads
+    inv = cfg.rope_theta ** (-torch.arange(0, d, 2, device=ids.device).double() / d)
+    angle = torch.outer(torch.arange(s, device=ids.device).double(), inv)
+    cos, sin = angle.cos(), angle.sin()
+    later = torch.ones(s, s, dtype=torch.bool, device=ids.device).triu(1)
+
+    def heads(x, rotate):
+        x = x.view(b, s, -1, d).transpose(1, 2)
+        if rotate:
+            x1, x2 = x.chunk(2, -1)
+            x = torch.cat((x1 * cos - x2 * sin, x2 * cos + x1 * sin), -1)
+        return x
+
+    x = p["embed_tokens.weight"][ids]
+    for i in range(cfg.n_layers):
+        w = {n: p["layers.%d.%s.weight" % (i, n)] for n in (
+            "input_layernorm", "self_attn.q_proj", "self_attn.k_proj", "self_attn.v_proj", "self_attn.o_proj",
+            "post_attention_layernorm", "mlp.gate_proj", "mlp.up_proj", "mlp.down_proj")}
+        h = norm(x, w["input_layernorm"])
+        q = heads(h @ w["self_attn.q_proj"].T, True)
+        k = heads(h @ w["self_attn.k_proj"].T, True)
+        v = heads(h @ w["self_attn.v_proj"].T, False)
+        o = []
+        for j in range(q.shape[1]):             # one head at a time: the scores are the large ones
+            g = j // (q.shape[1] // kv)
+            scores = (q[:, j] @ k[:, g].transpose(1, 2) / math.sqrt(d)).masked_fill(later, -math.inf)
+            o.append(scores.softmax(-1) @ v[:, g])
+        x = x + torch.cat(o, -1) @ w["self_attn.o_proj"].T
+        h = norm(x, w["post_attention_layernorm"])
+        x = x + (nn.functional.silu(h @ w["mlp.gate_proj"].T) * (h @ w["mlp.up_proj"].T)) @ w["mlp.down_proj"].T
+    x = norm(x, p["norm.weight"])
+    return x @ p.get("lm_head.weight", p["embed_tokens.weight"]).T
+
+
+def exact(case, seed):
+    tokens = case.get("batch", 0) * case.get("seq", 0)
+    if case["kind"] == "train" and tokens * case["vocab"] > 1.4e8:
+        return None                             # logits, their gradient and the scores of every layer at 8 bytes
+    state = prepare(case, seed)
+    if case["kind"] == "orthogonalise":
+        return _exact_newton_schulz(state["grad"])
+    if case["kind"] == "evaluate":
+        weights = {n: w.detach().double() for n, w in state["model"].named_parameters()}
+        with torch.no_grad():
+            return _exact_decoder(_decoder(case), weights, state["ids"])
+    if case["kind"] == "update":
+        grads = {"layers.%d.mats.%s.weight" % (i, n): g for i, layer in enumerate(state["grads"])
+                 for n, g in zip(_layer_shapes(case), layer)}
+        order = [dp.fqn for dp in state["owned"]]
+        plain, out = [], []
+    else:
+        owned = dmuon.get_owned_params(state["model"])
+        order = [dp.fqn for dp in owned]
+        plain = [n for n, p in state["model"].named_parameters() if hasattr(p, "to_local")]
+        leaves = {n: w.double().view(dp._orig_size).requires_grad_() for n, dp, w in zip(order, owned, state["weights"])}
+        leaves.update((n, w.double().requires_grad_()) for n, w in zip(plain, state["weights"][len(owned):]))
+        ids = state["ids"]
+        logits = _exact_decoder(_decoder(case), leaves, ids[:, :-1])
+        loss = nn.functional.cross_entropy(logits.flatten(0, 1), ids[:, 1:].flatten())
+        grads = dict(zip(leaves, torch.autograd.grad(loss, list(leaves.values()))))
+        out = [loss.detach()]
+    coef = 1.0
+    if case["clip"] > 0:
+        total = torch.stack([grads[n].double().norm() for n in order]).norm()
+        coef = torch.clamp(case["clip"] / (total + 1e-6), max=1.0)
+        out.append(total)
+    with torch.no_grad():
+        if case["kind"] == "update":
+            out += [grads[n].double() * coef for n in order]        # momentum after its first step
+        out += [_exact_muon(w.view(grads[n].shape), grads[n].double() * coef) for n, w in zip(order, state["weights"])]
+        out += [_exact_adamw(w.double(), grads[n]) for n, w in zip(plain, state["weights"][len(order):])]
+    return out
+
+
 # ---------------------------------------------------------------------------- what a pass cannot do without
 def _newton_schulz_flops(rows, cols, backend="gram"):
     """Five steps; a symmetric product counts half."""
