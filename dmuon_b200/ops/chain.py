@@ -1,0 +1,556 @@
+"""Newton-Schulz as one launch: plans for the product-chain kernel
+(``csrc/chain_sm100.cu``).
+
+A *group* is a batch of ``L`` matrices of one shape.  A *plan* covers one or more
+groups: it owns their work buffers, the encoded tensor maps, the list of products
+and the tile list, all on the device and reused by every call with the same
+shapes.  A call supplies only what changes: where the results go and the scale of
+the last product (plus the operands, written into ``plan.groups[i].X`` beforehand).
+
+The tile list is ordered product by product, all groups side by side; every entry
+names the number of finished warps its matrix must show before the tile may start
+(see the kernel source for why that cannot deadlock).
+"""
+from __future__ import annotations
+
+import ctypes
+import math
+import threading
+from collections import OrderedDict
+from dataclasses import dataclass
+from functools import lru_cache
+from typing import Optional, Sequence
+
+import numpy as np
+import torch
+
+from . import build as _build
+from . import gemm as G
+
+MAX_OPS = 76
+MAX_GROUPS = 16
+SMS = 148
+_KB = 64                      # inner elements per pipeline stage
+_SUM_COLS = 64                # columns of one entry of a sum of partial products
+WARPS_PER_TILE = 8            # epilogue warps per CTA: each reports a finished tile
+PAIR = 256                    # tile width that stands for CTA pairs on 256 x 256 tiles
+
+_VP, _LL, _I, _F = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_float
+
+
+class _Op(ctypes.Structure):
+    _fields_ = [
+        ("map_a", _I), ("map_b", _I), ("a_mn_major", _I), ("b_mn_major", _I), ("ab_fp16", _I),
+        ("M", _I), ("N", _I), ("K", _I), ("kb_per_split", _I), ("splits", _I), ("out_kind", _I), ("final_slot", _I),
+        ("alpha", _F), ("beta", _F), ("diag", _F), ("pad_", _I),
+        ("alpha_vec", _VP), ("C", _VP), ("D", _VP), ("partials", _VP),
+        ("ldc", _LL), ("ldd", _LL), ("strideC", _LL), ("strideD", _LL),
+    ]
+
+
+class _Final(ctypes.Structure):
+    _fields_ = [
+        ("C", _VP), ("D", _VP), ("C_tab", _VP), ("D_tab", _VP), ("D2_tab", _VP), ("alpha_vec", _VP),
+        ("ldc", _LL), ("ldd", _LL), ("ldd2", _LL), ("strideC", _LL), ("strideD", _LL),
+        ("alpha", _F), ("beta", _F), ("out_kind", _I), ("pad_", _I),
+    ]
+
+
+class _Map(ctypes.Structure):
+    _fields_ = [
+        ("base", _VP), ("rows", _LL), ("cols", _LL), ("batch", _LL), ("ld", _LL), ("batch_stride", _LL),
+        ("fp16", _I), ("box_cols", _I), ("box_rows", _I), ("pad_", _I),
+    ]
+
+
+class _Args(ctypes.Structure):
+    _fields_ = [
+        ("ops", _VP), ("maps", _VP), ("tab", _VP), ("counters", _VP), ("status", _VP),
+        ("n_ops", _I), ("n_maps", _I), ("total", _I), ("n_counters", _I), ("n_final", _I), ("bn", _I),
+        ("max_ctas", _I), ("pad_", _I),
+        ("fin", _Final * MAX_GROUPS),
+    ]
+
+
+@lru_cache(maxsize=None)
+def _lib():
+    lib = _build.load()
+    lib.dmuon_chain_encode_maps.argtypes = [ctypes.POINTER(_Map), _I, _VP]
+    lib.dmuon_chain_encode_maps.restype = _I
+    lib.dmuon_chain_launch.argtypes = [ctypes.POINTER(_Args), _VP]
+    lib.dmuon_chain_launch.restype = _I
+    return lib
+
+
+def fp16_prescale(m0: int, n0: int) -> float:
+    return float(2 ** round(math.log2(math.sqrt(min(m0, n0)))))
+
+
+# ---------------------------------------------------------------------------- the products of one group
+@dataclass
+class Product:
+    """``out = alpha * A B^T + beta * C + diag * I`` on named buffers of a group."""
+
+    A: str
+    B: str
+    out: str                        # "final": the caller's output
+    a_mn: bool = False
+    b_mn: bool = False
+    C: Optional[str] = None
+    alpha: float = 1.0
+    beta: float = 0.0
+    diag: float = 0.0
+    vec: Optional[str] = None       # per-matrix factor: "vec" or "vec2"
+    symmetric: bool = False
+    after: int = -1                 # index of the last product that has to be finished first (-1: none)
+
+
+def iteration_products(left: bool, coefs, restarts, formulation: str, h: float, with_vec: bool) -> list[Product]:
+    """The products of the iteration in issue order (the recurrences of
+    :mod:`dmuon_b200.optim.newton_schulz`); ``h`` is the host factor between the
+    stored operand and the normalised matrix, ``with_vec`` adds the per-matrix one."""
+    out: list[Product] = []
+
+    def add(**kw) -> int:
+        out.append(Product(**kw))
+        return len(out) - 1
+
+    def gram(X: str, dst: str, after: int) -> int:
+        return add(A=X, B=X, out=dst, a_mn=not left, b_mn=not left, alpha=h * h, vec="vec2" if with_vec else None,
+                   symmetric=True, after=after)
+
+    def apply(Q: str, X: str, dst: str, after: int, **kw) -> int:
+        if left:
+            return add(A=Q, B=X, out=dst, b_mn=True, after=after, **kw)
+        return add(A=X, B=Q, out=dst, after=after, **kw)
+
+    X, Xn = "X", "X2"
+    last = len(coefs) - 1
+    if formulation == "direct":
+        done = -1
+        for i, (a, b, c) in enumerate(coefs):
+            done = gram(X, "R", done)
+            done = add(A="R", B="R", out="P", C="R", alpha=c, beta=b, symmetric=True, after=done)
+            done = apply("P", X, "final" if i == last else Xn, done, C=X, beta=a)
+            X, Xn = Xn, X
+        return out
+
+    done = gram(X, "R", -1)
+    R, Rn = "R", "R2"
+    pool = ("Qa", "Qb", "P")
+    Q: Optional[str] = None
+    for i, (a, b, c) in enumerate(coefs):
+        if i in restarts and i != 0:
+            done = apply(Q, X, Xn, done)
+            X, Xn = Xn, X
+            done = gram(X, R, done)
+            Q = None
+        P = next(t for t in pool if t != Q)
+        done = add(A=R, B=R, out=P, C=R, alpha=c, beta=b, diag=a, symmetric=True, after=done)
+        more = i < last and (i + 1) not in restarts
+        after_p = done
+        if Q is None:
+            Q = P
+        else:
+            T = next(t for t in pool if t not in (Q, P))
+            done = add(A=P, B=Q, out=T, symmetric=True, after=after_p)
+            Q = T
+        if more:
+            # needs only P: runs beside the product above
+            done = add(A=R, B=P, out="RP", symmetric=True, after=after_p)
+            done = add(A="RP", B=P, out=Rn, symmetric=True, after=done)
+            R, Rn = Rn, R
+    apply(Q, X, "final", done, alpha=h, vec="vec" if with_vec else None)
+    return out
+
+
+# ---------------------------------------------------------------------------- groups and plans
+@dataclass(frozen=True)
+class GroupSpec:
+    L: int
+    m0: int
+    n0: int
+    dtype: torch.dtype
+    formulation: str
+    coefs: tuple
+    restarts: tuple
+    h: float
+    with_vec: bool
+
+    def __hash__(self) -> int:
+        # a key of every call: the nested coefficients are hashed once
+        h = self.__dict__.get("_hash")
+        if h is None:
+            h = hash((self.L, self.m0, self.n0, self.dtype, self.formulation, self.coefs, self.restarts, self.h,
+                      self.with_vec))
+            object.__setattr__(self, "_hash", h)
+        return h
+
+    @property
+    def left(self) -> bool:
+        return self.m0 <= self.n0
+
+    @property
+    def m(self) -> int:
+        return min(self.m0, self.n0)
+
+    @property
+    def n(self) -> int:
+        return max(self.m0, self.n0)
+
+
+@lru_cache(maxsize=4096)
+def _products_of(spec: GroupSpec) -> tuple[Product, ...]:
+    return tuple(iteration_products(spec.left, spec.coefs, spec.restarts, spec.formulation, spec.h, spec.with_vec))
+
+
+def tile_rows(bn: int) -> int:
+    return 256 if bn == PAIR else G.BM
+
+
+def _tiles(m: int, n: int, bn: int, symmetric: bool) -> np.ndarray:
+    """[T, 3] of (row tile, column tile, mirror)."""
+    bm = tile_rows(bn)
+    t = G.symmetric_tiles(m, bn, bm) if symmetric else G.dense_tiles(m, n, bn, bm)
+    return np.asarray(t, dtype=np.int64).reshape(-1, 3)
+
+
+def sym_tiles(specs: Sequence[GroupSpec], bn: int) -> int:
+    """Tiles of one symmetric product of every group."""
+    return sum(s.L * len(G.symmetric_tiles(s.m, bn, tile_rows(bn))) for s in specs)
+
+
+def fits(specs: Sequence[GroupSpec]) -> bool:
+    """Within what a plan's tables can express, matrices the kernels take."""
+    if len(specs) > MAX_GROUPS or sum(s.L for s in specs) > 4096:
+        return False
+    if any(s.m0 % 8 or s.n0 % 8 or s.m < 8 or not s.coefs for s in specs):
+        return False
+    # a Gram product that is split over K counts twice
+    split = choose_bn(specs) != PAIR
+    return sum(len(p) + split * sum(q.symmetric and q.A in ("X", "X2") for q in p) for p in map(_products_of, specs)) <= MAX_OPS
+
+
+def choose_bn(specs: Sequence[GroupSpec]) -> int:
+    """CTA pairs once a symmetric product of all groups has a 256 x 256 tile for each
+    of them.  Below that, half-width tiles while 128-wide ones leave half of the SMs
+    without work: an SM is fed 64 bytes per clock, so more SMs with less each finish
+    sooner."""
+    if sym_tiles(specs, PAIR) * 2 >= SMS:
+        return PAIR
+    return 64 if sym_tiles(specs, 128) * 2 <= SMS else 128
+
+
+def gram_splits(spec: GroupSpec, bn: int, tiles_all: int) -> tuple[int, int]:
+    """(splits, k-blocks per split) of the Gram product: as many splits as keep
+    the SMs busy, each with at least eight k-blocks to amortise its partial tile.
+    CTA pairs are taken only where there are tiles enough."""
+    num_kb = -(-spec.n // _KB)
+    splits = 1 if bn == PAIR else max(1, min(SMS // max(1, tiles_all), num_kb // 8, 16))
+    per = -(-num_kb // splits)
+    return -(-num_kb // per), per
+
+
+class Arena:
+    """Work memory of one stream.  Plans of a stream use it one after the other (the
+    operands are written, the chain runs, the result leaves), so they share it; the
+    lock spans those steps on the host."""
+
+    def __init__(self, nbytes: int, device):
+        self.lock = threading.RLock()
+        self.buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        self.used = 0
+
+    def take(self, shape, dtype) -> torch.Tensor:
+        n = math.prod(shape) * torch.empty(0, dtype=dtype).element_size()
+        t = self.buf[self.used : self.used + n].view(dtype).view(shape)
+        self.used += -(-n // 1024) * 1024
+        return t
+
+
+def _buffer_shapes(spec: GroupSpec, splits: int) -> dict:
+    L, m = spec.L, spec.m
+    names = ("R", "P") if spec.formulation == "direct" else ("R", "R2", "RP", "P", "Qa", "Qb")
+    out = {b: ((L, m, m), spec.dtype) for b in names}
+    out["X"] = out["X2"] = ((L, spec.m0, spec.n0), spec.dtype)
+    if splits > 1:
+        out["partials"] = ((L * splits, m, m), torch.float32)
+    return out
+
+
+def plan_bytes(specs: Sequence[GroupSpec]) -> int:
+    bn = choose_bn(specs)
+    tiles = sym_tiles(specs, bn)
+    total = 0
+    for s in specs:
+        for shape, dtype in _buffer_shapes(s, gram_splits(s, bn, tiles)[0]).values():
+            n = math.prod(shape) * (4 if dtype == torch.float32 else 2)
+            total += -(-n // 1024) * 1024
+    return total
+
+
+class Group:
+    """Work buffers of one group."""
+
+    def __init__(self, spec: GroupSpec, splits: int, arena: Arena):
+        self.spec = spec
+        arena_of = _buffer_shapes(spec, splits)
+        self.buffers = {name: arena.take(shape, dtype) for name, (shape, dtype) in arena_of.items()}
+        self.X = self.buffers["X"]
+        self.partials: Optional[torch.Tensor] = self.buffers.get("partials")
+
+
+def build_entries(specs: Sequence[GroupSpec], bn: int):
+    """Products and tile list of a plan, without touching a device.
+
+    Returns ``(ops, entries)``: ``ops`` are ``(group, Product, splits, kb_per_split, is_sum)``
+    and ``entries`` is an int32 array ``[T, 4]`` in the kernel's packing."""
+    per_group = [_products_of(s) for s in specs]
+    tiles_all = sym_tiles(specs, bn)
+    splits = [gram_splits(s, bn, tiles_all) for s in specs]
+    first_matrix = np.cumsum([0] + [s.L for s in specs])
+    ops: list = []
+    chunks: list[np.ndarray] = []
+    # finished warps of one matrix of group g after product i (all tiles of products 0..i)
+    total = [0] * len(specs)
+    upto: list[list[int]] = [[] for _ in specs]
+
+    def emit(g: int, op: int, tiles: np.ndarray, want: int, split: int = 0) -> None:
+        L = specs[g].L
+        b = np.repeat(np.arange(L), len(tiles))
+        t = np.tile(tiles, (L, 1))
+        e = np.empty((len(b), 4), dtype=np.int64)
+        e[:, 0] = op | (t[:, 2] << 8) | (split << 16)
+        e[:, 1] = t[:, 0] | (t[:, 1] << 16)
+        e[:, 2] = b | ((first_matrix[g] + b) << 16)
+        e[:, 3] = want
+        chunks.append(e)
+        total[g] += len(tiles) * WARPS_PER_TILE * (2 if bn == PAIR else 1)
+
+    for i in range(max(len(p) for p in per_group)):
+        for g, s in enumerate(specs):
+            if i >= len(per_group[g]):
+                continue
+            pr = per_group[g][i]
+            want = upto[g][pr.after] if pr.after >= 0 else 0
+            is_gram = pr.symmetric and pr.A == pr.B and pr.A in ("X", "X2")
+            ns, per = splits[g] if is_gram else (1, 0)
+            rows = s.m if pr.symmetric else s.m0
+            cols = s.m if pr.symmetric else s.n0
+            tiles = _tiles(rows, cols, bn, pr.symmetric)
+            if ns > 1:
+                plain = tiles.copy()
+                plain[:, 2] = 0
+                ops.append((g, pr, ns, per, False))
+                for k in range(ns):
+                    emit(g, len(ops) - 1, plain, want, k)
+                ops.append((g, pr, ns, 0, True))
+                emit(g, len(ops) - 1, _tiles(rows, cols, _SUM_COLS, True), total[g])
+            else:
+                ops.append((g, pr, 1, 0, False))
+                emit(g, len(ops) - 1, tiles, want)
+            upto[g].append(total[g])
+    entries = np.concatenate(chunks) if chunks else np.zeros((0, 4), dtype=np.int64)
+    # the packing holds 31 bits per word; the sign bit of the first word marks the end of the list
+    return ops, (entries & 0xFFFFFFFF).astype(np.uint32).view(np.int32)
+
+
+class Plan:
+    def __init__(self, specs: Sequence[GroupSpec], device: torch.device, arena: Arena):
+        self.specs = tuple(specs)
+        self.device = device
+        self.bn = choose_bn(self.specs)
+        self.arena = arena
+        self.lock = arena.lock
+        tiles = sym_tiles(self.specs, self.bn)
+        arena.used = 0
+        self.groups = [Group(s, gram_splits(s, self.bn, tiles)[0], arena) for s in self.specs]
+        self.n_matrices = sum(s.L for s in self.specs)
+        self.first = [0]
+        for s in self.specs:
+            self.first.append(self.first[-1] + s.L)
+        n = self.n_matrices
+        # ticket, exits, one counter per matrix, then the sums of squares: all cleared by the kernel itself
+        self.counters = torch.zeros(2 + 2 * n, dtype=torch.int32, device=device)
+        self.sumsq = self.counters[2 + n :].view(torch.float32)
+        self.vec = torch.empty(n, dtype=torch.float32, device=device)
+        self.vec2 = torch.empty(n, dtype=torch.float32, device=device)
+        # the power of two that keeps fp16 operands clear of the subnormals, per matrix
+        self.k = torch.tensor([fp16_prescale(s.m0, s.n0) for s in self.specs for _ in range(s.L)], device=device)
+        self.dirty = False          # a call was abandoned half-way: the counters have to be cleared
+        self.pinned = False         # captured in a CUDA graph
+        ops, entries = build_entries(self.specs, self.bn)
+        assert len(ops) <= MAX_OPS
+        self._encode(ops)
+        self.tab = torch.from_numpy(entries.copy()).to(device)
+        self.total = int(entries.shape[0])
+        a = _Args()
+        a.ops, a.maps, a.tab = self._ops.data_ptr(), self._maps.data_ptr(), self.tab.data_ptr()
+        a.counters, a.status = self.counters.data_ptr(), G.status_buffer(device).data_ptr()
+        a.n_ops, a.n_maps, a.total = self.n_ops, self.n_maps, self.total
+        a.n_counters, a.n_final, a.bn = self.counters.numel(), len(self.specs), self.bn
+        self._args = a
+
+    def _encode(self, ops) -> None:
+        maps: list[_Map] = []
+        index: dict[tuple, int] = {}
+
+        def map_of(g: int, name: str, mn: bool, rows_per_tile: int) -> int:
+            box = (64, _KB) if mn else (_KB, rows_per_tile)
+            key = (g, name, box)
+            if key not in index:
+                t = self.groups[g].buffers[name]
+                L, r, c = t.shape
+                m = _Map()
+                m.base, m.rows, m.cols, m.batch, m.ld, m.batch_stride = t.data_ptr(), r, c, L, c, r * c
+                m.fp16, m.box_cols, m.box_rows = int(t.dtype == torch.float16), box[0], box[1]
+                index[key] = len(maps)
+                maps.append(m)
+            return index[key]
+
+        arr = (_Op * len(ops))()
+        for i, (g, pr, ns, per, is_sum) in enumerate(ops):
+            s, grp = self.specs[g], self.groups[g]
+            o = arr[i]
+            o.M = s.m if pr.symmetric else s.m0
+            o.N = s.m if pr.symmetric else s.n0
+            o.K = s.n if (pr.symmetric and pr.A in ("X", "X2")) else s.m
+            o.a_mn_major, o.b_mn_major = int(pr.a_mn), int(pr.b_mn)
+            o.ab_fp16 = int(s.dtype == torch.float16)
+            o.final_slot, o.splits, o.kb_per_split = -1, ns, per
+            o.map_a = -1 if is_sum else map_of(g, pr.A, pr.a_mn, G.BM)
+            o.map_b = -1 if is_sum else map_of(g, pr.B, pr.b_mn, min(self.bn, G.BM))
+            if ns > 1 and not is_sum:
+                o.alpha, o.out_kind = 1.0, 2
+                o.D, o.ldd, o.strideD = grp.partials.data_ptr(), s.m, s.m * s.m
+                continue
+            o.alpha, o.beta, o.diag = pr.alpha, pr.beta, pr.diag
+            o.out_kind = G._OUT_KIND[s.dtype]
+            if pr.vec is not None:
+                o.alpha_vec = (self.vec if pr.vec == "vec" else self.vec2).data_ptr() + 4 * self.first[g]
+            if is_sum:
+                o.partials = grp.partials.data_ptr()
+            if pr.C is not None:
+                c = grp.buffers[pr.C]
+                o.C, o.ldc, o.strideC = c.data_ptr(), c.stride(1), c.stride(0)
+            if pr.out == "final":
+                o.final_slot = g
+            else:
+                d = grp.buffers[pr.out]
+                o.D, o.ldd, o.strideD = d.data_ptr(), d.stride(1), d.stride(0)
+        n = len(maps)
+        marr = (_Map * n)(*maps)
+        raw = ctypes.create_string_buffer(128 * n + 64)
+        base = (ctypes.addressof(raw) + 63) & ~63
+        rc = _lib().dmuon_chain_encode_maps(marr, n, base)
+        if rc != 0:
+            raise RuntimeError(f"dmuon_chain_encode_maps failed with code {rc}")
+        enc = np.frombuffer(ctypes.string_at(base, 128 * n), dtype=np.uint8).copy()
+        self._maps = torch.from_numpy(enc).to(self.device)
+        self._ops = torch.from_numpy(np.frombuffer(bytes(arr), dtype=np.uint8).copy()).to(self.device)
+        self.n_ops, self.n_maps = len(ops), n
+        self._finals = {g: pr for g, pr, *_ in ops if pr.out == "final"}
+
+    def begin(self) -> None:
+        """Call before the sums of squares are accumulated."""
+        if self.dirty:
+            self.counters.zero_()
+        self.dirty = True
+
+    def run(self, finals: Sequence[dict]) -> None:
+        """Launch the chain on the current stream.  ``finals[g]``: ``out`` (a
+        ``[L, m0, n0]`` tensor) or ``out_tab`` / ``c_tab`` / ``out2_tab`` (device tables
+        of addresses, multiples of 16 bytes) with ``out_dtype``; ``alpha`` multiplies the plan's own factor."""
+        a = self._args
+        for g, f in enumerate(finals):
+            s, pr, fin = self.specs[g], self._finals[g], a.fin[g]
+            fin.alpha = float(f.get("alpha", 1.0)) * pr.alpha
+            fin.alpha_vec = self.vec.data_ptr() + 4 * self.first[g] if pr.vec is not None else None
+            fin.C = fin.C_tab = fin.D = fin.D_tab = fin.D2_tab = None
+            fin.ldc = fin.ldd = fin.ldd2 = s.n0
+            fin.strideC = fin.strideD = s.m0 * s.n0
+            fin.beta = 0.0
+            out = f.get("out")
+            if out is not None:
+                fin.D, fin.out_kind = out.data_ptr(), G._OUT_KIND[out.dtype]
+                if pr.C is not None:
+                    assert out.dtype == s.dtype
+                    fin.C, fin.beta = self.groups[g].buffers[pr.C].data_ptr(), pr.beta
+                continue
+            assert pr.C is None
+            fin.D_tab, fin.out_kind = f["out_tab"].data_ptr(), G._OUT_KIND[f["out_dtype"]]
+            if f.get("c_tab") is not None:
+                fin.C_tab, fin.beta = f["c_tab"].data_ptr(), float(f["beta"])
+            if f.get("out2_tab") is not None:
+                fin.D2_tab = f["out2_tab"].data_ptr()
+        stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(self.device.index))
+        rc = _lib().dmuon_chain_launch(ctypes.byref(a), stream)
+        if rc != 0:
+            raise RuntimeError(f"dmuon_chain_launch failed with code {rc}")
+        self.dirty = False
+
+
+# ---------------------------------------------------------------------------- plans that are kept
+#: what the work buffers of one plan may take together
+MAX_PLAN_BYTES = 6 << 30
+MAX_PLANS = 256
+MAX_ARENAS = 8
+_plans: "OrderedDict[tuple, Plan]" = OrderedDict()
+_arenas: "OrderedDict[tuple, Arena]" = OrderedDict()
+_lock = threading.RLock()
+
+
+@lru_cache(maxsize=4096)
+def possible(specs: tuple[GroupSpec, ...]) -> bool:
+    """These groups can be one plan."""
+    return fits(specs) and plan_bytes(specs) <= MAX_PLAN_BYTES
+
+
+def plan_for(specs: Sequence[GroupSpec], device: torch.device) -> Optional[Plan]:
+    """The plan of these groups for the current stream (work memory is never shared
+    between streams).  While a CUDA graph is captured nothing can be uploaded:
+    then a plan that an earlier call made on another stream is taken and kept for
+    good, and ``None`` is returned if there is none."""
+    sig = (tuple(specs), device.index)
+    if torch.cuda.is_current_stream_capturing():
+        with _lock:
+            for k, p in _plans.items():
+                if k[0] == sig:
+                    p.pinned = True
+                    return p
+        return None
+    where = (device.index, torch._C._cuda_getCurrentRawStream(device.index))
+    key = (sig, where)
+    with _lock:
+        p = _plans.get(key)
+        if p is not None:
+            _plans.move_to_end(key)
+            return p
+        need = plan_bytes(specs)
+        arena = _arenas.get(where)
+        if arena is None or arena.buf.numel() < need:
+            # plans made on the smaller memory go (a captured one keeps its own alive)
+            _drop(lambda k, q: k[1] == where and not q.pinned)
+            _arenas.pop(where, None)
+            arena = None
+            arena = _arenas[where] = Arena(need, device)
+        _arenas.move_to_end(where)
+        while len(_arenas) > MAX_ARENAS:
+            old, _ = _arenas.popitem(last=False)
+            _drop(lambda k, q: k[1] == old and not q.pinned)
+        if len(_plans) >= MAX_PLANS:
+            oldest = next((k for k, q in _plans.items() if not q.pinned), None)
+            _plans.pop(oldest, None)
+        p = _plans[key] = Plan(specs, device, arena)
+        return p
+
+
+def _drop(which) -> None:
+    for k in [k for k, q in _plans.items() if which(k, q)]:
+        del _plans[k]
+
+
+def release() -> None:
+    with _lock:
+        _plans.clear()
+        _arenas.clear()

@@ -25,16 +25,12 @@
 #include <atomic>
 #include <mutex>
 
+#include "gemm_epilogue.cuh"
 #include "gemm_sm100.cuh"
 #include "ptx_sm100.cuh"
+#include "tensor_map.cuh"
 
 namespace dmuon {
-
-constexpr int BM = 128;
-constexpr int BK = 64;       // 64 two-byte elements = one 128-byte swizzle row
-constexpr int UMMA_K = 16;
-constexpr int kThreads = 192;
-constexpr int kBlockBytes = 64 * 128;  // one 64 x 64 swizzled block (MN-major staging)
 
 template <int BN>
 struct Cfg {
@@ -46,149 +42,6 @@ struct Cfg {
   static constexpr int kBarBytes = 256;
   static constexpr int kSmemBytes = kStages * kStageBytes + kBarBytes + 1024;
 };
-
-struct KParams {
-  int M, N, K, batch;
-  const int4* tile_tab;
-  int tiles_per_batch;
-  int a_mn_major, b_mn_major, ab_fp16;
-  float alpha, beta, diag;
-  const float* alpha_vec;
-  const void* C;
-  void* D;
-  void* D2;
-  const void* const* C_tab;
-  void* const* D_tab;
-  void* const* D2_tab;
-  long long ldc, ldd, ldd2;
-  long long strideC, strideD, strideD2;
-  int out_kind;
-  const int* b_ready;
-  int b_ready_epoch;
-  int* status;
-  int d2_multimem;
-};
-
-// ---- epilogue helpers -------------------------------------------------------
-
-template <typename T>
-__device__ __forceinline__ float to_f32(T x);
-template <>
-__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 x) { return __bfloat162float(x); }
-template <>
-__device__ __forceinline__ float to_f32<__half>(__half x) { return __half2float(x); }
-template <>
-__device__ __forceinline__ float to_f32<float>(float x) { return x; }
-
-template <typename T>
-__device__ __forceinline__ T from_f32(float x);
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
-template <>
-__device__ __forceinline__ __half from_f32<__half>(float x) { return __float2half_rn(x); }
-template <>
-__device__ __forceinline__ float from_f32<float>(float x) { return x; }
-
-template <typename T>
-__device__ __forceinline__ void load_row32(const T* src, float (&c)[32], int nvalid, bool vec) {
-  if (vec && nvalid == 32) {
-    constexpr int kPerVec = 16 / sizeof(T);
-    const uint4* s4 = reinterpret_cast<const uint4*>(src);
-#pragma unroll
-    for (int i = 0; i < 32 / kPerVec; ++i) {
-      uint4 raw = s4[i];
-      const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-      for (int j = 0; j < kPerVec; ++j) c[i * kPerVec + j] = to_f32<T>(e[j]);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) c[j] = (j < nvalid) ? to_f32<T>(src[j]) : 0.f;
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void store_row32(T* dst, const float (&v)[32], int nvalid, bool vec) {
-  if (vec && nvalid == 32) {
-    constexpr int kPerVec = 16 / sizeof(T);
-    uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-    for (int i = 0; i < 32 / kPerVec; ++i) {
-      uint4 raw;
-      T* e = reinterpret_cast<T*>(&raw);
-#pragma unroll
-      for (int j = 0; j < kPerVec; ++j) e[j] = from_f32<T>(v[i * kPerVec + j]);
-      d4[i] = raw;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j < nvalid) dst[j] = from_f32<T>(v[j]);
-  }
-}
-
-// bf16 row chunk to a multicast address: every rank's copy of the buffer
-// receives it (multimem.st through the switch).  The host only selects this
-// path when every row start is 16-byte aligned and N is a multiple of 8.
-__device__ __forceinline__ void store_row32_multicast(__nv_bfloat16* mc_dst, const float (&v)[32], int nvalid) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (i * 8 < nvalid) {
-      uint4 raw;
-      __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&raw);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) e[j] = __float2bfloat16_rn(v[i * 8 + j]);
-      multimem_st_16B(mc_dst + i * 8, raw);
-    }
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void store_col32(T* dst, long long ld, const float (&v)[32], int nvalid) {
-  // dst points at element (col0, row) of the transposed tile; consecutive
-  // lanes hold consecutive rows, so each store instruction is contiguous
-  // across the warp.
-#pragma unroll
-  for (int j = 0; j < 32; ++j)
-    if (j < nvalid) dst[static_cast<long long>(j) * ld] = from_f32<T>(v[j]);
-}
-
-template <typename T>
-__device__ __forceinline__ void epilogue_chunk(const KParams& p, const T* Cb, T* Db,
-                                               __nv_bfloat16* D2b, float (&v)[32], int row, int col0,
-                                               bool mirror) {
-  const int nvalid = min(32, p.N - col0);
-  const bool row_ok = row < p.M;
-  if (p.beta != 0.f && row_ok) {
-    float c[32];
-    const T* src = Cb + static_cast<long long>(row) * p.ldc + col0;
-    const bool vec = ((p.ldc * sizeof(T)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(Cb) & 15) == 0);
-    load_row32<T>(src, c, nvalid, vec);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = fmaf(p.beta, c[j], v[j]);
-  }
-  if (p.diag != 0.f) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (col0 + j == row) v[j] += p.diag;
-  }
-  if (!row_ok) return;
-  {
-    T* dst = Db + static_cast<long long>(row) * p.ldd + col0;
-    const bool vec = ((p.ldd * sizeof(T)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(Db) & 15) == 0);
-    store_row32<T>(dst, v, nvalid, vec);
-    if (mirror) store_col32<T>(Db + static_cast<long long>(col0) * p.ldd + row, p.ldd, v, nvalid);
-  }
-  if (D2b != nullptr && p.d2_multimem) {
-    store_row32_multicast(D2b + static_cast<long long>(row) * p.ldd2 + col0, v, nvalid);
-  } else if (D2b != nullptr) {
-    __nv_bfloat16* dst = D2b + static_cast<long long>(row) * p.ldd2 + col0;
-    const bool vec = ((p.ldd2 * 2) % 16 == 0) && ((reinterpret_cast<uintptr_t>(D2b) & 15) == 0);
-    store_row32<__nv_bfloat16>(dst, v, nvalid, vec);
-    if (mirror)
-      store_col32<__nv_bfloat16>(D2b + static_cast<long long>(col0) * p.ldd2 + row, p.ldd2, v, nvalid);
-  }
-}
 
 // ---- kernel -------------------------------------------------------------------
 
@@ -358,37 +211,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         break;
       }
       tc_fence_after_sync();
-      const int row = m0 + q * 32 + lane;
-      const char* Cb = reinterpret_cast<const char*>(p.C_tab ? p.C_tab[b] : p.C);
-      char* Db = reinterpret_cast<char*>(p.D_tab ? p.D_tab[b] : p.D);
-      __nv_bfloat16* D2b = reinterpret_cast<__nv_bfloat16*>(p.D2_tab ? p.D2_tab[b] : p.D2);
-      const int esz = (p.out_kind == 2) ? 4 : 2;
-      if (!p.C_tab && Cb) Cb += static_cast<long long>(b) * p.strideC * esz;
-      if (!p.D_tab) Db += static_cast<long long>(b) * p.strideD * esz;
-      if (!p.D2_tab && D2b) D2b += static_cast<long long>(b) * p.strideD2;
-      const float alpha = p.alpha_vec ? p.alpha * p.alpha_vec[b] : p.alpha;
-      for (int c = 0; c < BN; c += 32) {
-        const int col0 = n0 + c;
-        if (col0 >= p.N) break;  // uniform across the warp
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                          static_cast<uint32_t>(acc * BN + c),
-                      r);
-        tmem_ld_wait();
-        float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = alpha * __uint_as_float(r[j]);
-        if (p.out_kind == 0) {
-          epilogue_chunk<__nv_bfloat16>(p, reinterpret_cast<const __nv_bfloat16*>(Cb),
-                                        reinterpret_cast<__nv_bfloat16*>(Db), D2b, v, row, col0, mirror);
-        } else if (p.out_kind == 1) {
-          epilogue_chunk<__half>(p, reinterpret_cast<const __half*>(Cb), reinterpret_cast<__half*>(Db),
-                                 D2b, v, row, col0, mirror);
-        } else {
-          epilogue_chunk<float>(p, reinterpret_cast<const float*>(Cb), reinterpret_cast<float*>(Db), D2b,
-                                v, row, col0, mirror);
-        }
-      }
+      epilogue_rows32(p, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN),
+                      m0 + q * 32 + lane, n0, BN, b, mirror);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty0 + 8 * acc);
@@ -593,35 +417,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         break;
       }
       tc_fence_after_sync();
-      const int row = m0 + q * 32 + lane;
-      const char* Cb = reinterpret_cast<const char*>(p.C_tab ? p.C_tab[b] : p.C);
-      char* Db = reinterpret_cast<char*>(p.D_tab ? p.D_tab[b] : p.D);
-      __nv_bfloat16* D2b = reinterpret_cast<__nv_bfloat16*>(p.D2_tab ? p.D2_tab[b] : p.D2);
-      const int esz = (p.out_kind == 2) ? 4 : 2;
-      if (!p.C_tab && Cb) Cb += static_cast<long long>(b) * p.strideC * esz;
-      if (!p.D_tab) Db += static_cast<long long>(b) * p.strideD * esz;
-      if (!p.D2_tab && D2b) D2b += static_cast<long long>(b) * p.strideD2;
-      const float alpha = p.alpha_vec ? p.alpha * p.alpha_vec[b] : p.alpha;
-      for (int c = 0; c < BNp; c += 32) {
-        const int col0 = n0 + c;
-        if (col0 >= p.N) break;
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BNp + c), r);
-        tmem_ld_wait();
-        float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = alpha * __uint_as_float(r[j]);
-        if (p.out_kind == 0) {
-          epilogue_chunk<__nv_bfloat16>(p, reinterpret_cast<const __nv_bfloat16*>(Cb),
-                                        reinterpret_cast<__nv_bfloat16*>(Db), D2b, v, row, col0, mirror);
-        } else if (p.out_kind == 1) {
-          epilogue_chunk<__half>(p, reinterpret_cast<const __half*>(Cb), reinterpret_cast<__half*>(Db), D2b, v,
-                                 row, col0, mirror);
-        } else {
-          epilogue_chunk<float>(p, reinterpret_cast<const float*>(Cb), reinterpret_cast<float*>(Db), D2b, v, row,
-                                col0, mirror);
-        }
-      }
+      epilogue_rows32(p, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BNp),
+                      m0 + q * 32 + lane, n0, BNp, b, mirror);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty0 + 8 * acc, 0));   // the leader's barrier
@@ -694,39 +491,6 @@ __device__ __forceinline__ bool poll_ge_bounded(volatile uint32_t* ctr, uint32_t
         *abort_flag = 1;
         return false;
       }
-    }
-  }
-}
-
-// One warp's share (32 accumulator rows) of a 256-column output tile.
-__device__ __forceinline__ void epilogue_rows32(const KParams& p, uint32_t tmem_addr, int row, int n0, int b,
-                                                bool mirror) {
-  const char* Cb = reinterpret_cast<const char*>(p.C_tab ? p.C_tab[b] : p.C);
-  char* Db = reinterpret_cast<char*>(p.D_tab ? p.D_tab[b] : p.D);
-  __nv_bfloat16* D2b = reinterpret_cast<__nv_bfloat16*>(p.D2_tab ? p.D2_tab[b] : p.D2);
-  const int esz = (p.out_kind == 2) ? 4 : 2;
-  if (!p.C_tab && Cb) Cb += static_cast<long long>(b) * p.strideC * esz;
-  if (!p.D_tab) Db += static_cast<long long>(b) * p.strideD * esz;
-  if (!p.D2_tab && D2b) D2b += static_cast<long long>(b) * p.strideD2;
-  const float alpha = p.alpha_vec ? p.alpha * p.alpha_vec[b] : p.alpha;
-  for (int c = 0; c < 256; c += 32) {
-    const int col0 = n0 + c;
-    if (col0 >= p.N) break;  // uniform across the warp
-    uint32_t r[32];
-    tmem_ld_32x32(tmem_addr + static_cast<uint32_t>(c), r);
-    tmem_ld_wait();
-    float v[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = alpha * __uint_as_float(r[j]);
-    if (p.out_kind == 0) {
-      epilogue_chunk<__nv_bfloat16>(p, reinterpret_cast<const __nv_bfloat16*>(Cb),
-                                    reinterpret_cast<__nv_bfloat16*>(Db), D2b, v, row, col0, mirror);
-    } else if (p.out_kind == 1) {
-      epilogue_chunk<__half>(p, reinterpret_cast<const __half*>(Cb), reinterpret_cast<__half*>(Db), D2b, v, row,
-                             col0, mirror);
-    } else {
-      epilogue_chunk<float>(p, reinterpret_cast<const float*>(Cb), reinterpret_cast<float*>(Db), D2b, v, row,
-                            col0, mirror);
     }
   }
 }
@@ -974,7 +738,7 @@ gemm_tcgen05_quad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       if (!filler) {
         const int row = m_blk * 256 + 128 * static_cast<int>(half) + q * 32 + lane;
         epilogue_rows32(p, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BNp), row,
-                        n_blk * BNp, b, mirror);
+                        n_blk * BNp, BNp, b, mirror);
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -1001,43 +765,6 @@ gemm_tcgen05_quad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 }
 
 // ---- host side ------------------------------------------------------------------
-
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                              CUtensorMapFloatOOBfill);
-
-static EncodeFn get_encode_fn() {
-  static EncodeFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeFn>(sym);
-  });
-  return fn;
-}
-
-// Tensor map over a batched row-major matrix [batch][rows][cols] of 2-byte
-// elements; the box is box_cols x box_rows x 1 with 128-byte swizzle.
-static int make_map(CUtensorMap* map, const void* base, bool fp16, long long cols, long long rows,
-                    long long batch, long long ld, long long batch_stride, int box_cols, int box_rows) {
-  EncodeFn enc = get_encode_fn();
-  if (enc == nullptr) return -2;
-  cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows),
-                        static_cast<cuuint64_t>(batch)};
-  long long bs = (batch > 1 && batch_stride > 0) ? batch_stride : rows * ld;
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(bs) * 2};
-  cuuint32_t box[3] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows), 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(map, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
-                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -3;
-}
 
 static std::atomic<long long> g_launches{0};
 

@@ -92,6 +92,18 @@ __global__ void norm_scales_kernel(const DmuonNormArgs a) {
   }
 }
 
+__global__ void rescale_kernel(const DmuonRescaleArgs a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.n) {
+    const float s = 1.f / (sqrtf(a.sumsq[i]) + a.eps);
+    const float k = a.k[i];
+    const float v = a.fresh ? 1.f / k : s / a.prescale[i];
+    a.vec[i] = v;
+    a.vec2[i] = v * v;
+    a.prescale[i] = s * k;
+  }
+}
+
 // ---------------------------------------------------------------- AdamW
 template <typename TP, typename TG, typename TS>
 __global__ void __launch_bounds__(kBlock) adamw_kernel(const DmuonAdamWArgs a) {
@@ -203,7 +215,8 @@ __global__ void __launch_bounds__(kBlock) cast_kernel(const DmuonCastArgs a) {
   const TS* s = reinterpret_cast<const TS*>(a.src[t]);
   TD* d = reinterpret_cast<TD*>(a.dst[t]);
   const long long n = a.numel[t];
-  const float c = a.scale ? a.scale[a.slot[t]] : 1.f;
+  float c = a.scale ? a.scale[a.slot[t]] : 1.f;
+  if (a.sumsq) c = a.norm_num / (sqrtf(a.sumsq[a.slot[t]]) + a.norm_eps);
   const bool vec = aligned16(s) && aligned16(d);
   const long long nvec = vec ? (n / kVec) : 0;
   const long long stride = static_cast<long long>(gridDim.x) * kBlock;
@@ -253,6 +266,14 @@ extern "C" int dmuon_norm_scales(const DmuonNormArgs* a, void* stream_v) {
   if (a->n <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
   norm_scales_kernel<<<(a->n + 127) / 128, 128, 0, st>>>(*a);
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int dmuon_rescale(const DmuonRescaleArgs* a, void* stream_v) {
+  if (a->n <= 0) return 0;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
+  rescale_kernel<<<(a->n + 127) / 128, 128, 0, st>>>(*a);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

@@ -32,6 +32,21 @@ struct DmuonPrologueArgs {
   const float* xscale;
 };
 
+// Scales of fp16 Gram operands that were stored with a factor known before the norm:
+//   s = 1 / (sqrt(sumsq) + eps);  vec = s / prescale (the products' correction), vec2 = vec^2,
+//   prescale = s * k (what the matrix is stored with next time)
+// fresh: the operand will be stored with the new prescale itself, so vec = 1 / k.
+struct DmuonRescaleArgs {
+  const float* sumsq;
+  const float* k;
+  float* prescale;
+  float* vec;
+  float* vec2;
+  int n;
+  int fresh;
+  float eps;
+};
+
 // scale[i] = 1 / (sqrt(sumsq[i]) + eps), scale2[i] = scale[i]^2
 struct DmuonNormArgs {
   const float* sumsq;
@@ -79,10 +94,14 @@ struct DmuonCastArgs {
   int n;
   int src_dtype, dst_dtype;
   const float* scale;                 // optional per-slot device scales
+  // optional instead of `scale`: the per-slot scale is norm_num / (sqrt(sumsq[slot]) + norm_eps)
+  const float* sumsq;
+  float norm_num, norm_eps;
 };
 
 int dmuon_muon_prologue(const DmuonPrologueArgs* a, void* stream);
 int dmuon_norm_scales(const DmuonNormArgs* a, void* stream);
+int dmuon_rescale(const DmuonRescaleArgs* a, void* stream);
 int dmuon_adamw(const DmuonAdamWArgs* a, void* stream);
 int dmuon_clip_sumsq(const DmuonClipArgs* a, void* stream);
 int dmuon_clip_scale(const DmuonClipArgs* a, void* stream);

@@ -83,6 +83,38 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
+// Bounded wait that also makes visible what ANOTHER CTA of the cluster stored into
+// this CTA's shared memory before it arrived (the plain form acquires for the CTA).
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+__device__ __forceinline__ bool mbar_wait_cluster_bounded(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try_wait_cluster(bar, parity)) return true;
+  const long long t0 = clock64();
+  uint32_t spins = 0;
+  while (true) {
+    if (mbar_try_wait_cluster(bar, parity)) return true;
+    if ((++spins & 63u) == 0u) {
+      if (*abort_flag) return false;
+      if (clock64() - t0 > kWaitBudgetCycles) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+}
+
 // Same with a caller-chosen budget (kernels whose progress depends on another
 // GPU wait as long as the cross-GPU flag waits do).
 __device__ __forceinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag,
@@ -291,6 +323,12 @@ __device__ __forceinline__ void bulk_copy_s2cluster(uint32_t dst_cluster, uint32
       : "memory");
 }
 
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, const int4& v) {
+  asm volatile("st.shared::cluster.v4.s32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(v.x), "r"(v.y), "r"(v.z),
+               "r"(v.w)
+               : "memory");
+}
+
 // A 32-bit progress counter in another CTA's shared memory (monotonic, so a
 // reader can never confuse two rounds the way a one-bit phase could).
 __device__ __forceinline__ void st_release_cluster_u32(uint32_t cluster_addr, uint32_t v) {
@@ -357,6 +395,10 @@ __device__ __forceinline__ void bulk_wait_group() {
 
 __device__ __forceinline__ void fence_proxy_async_all() {
   asm volatile("fence.proxy.async;" ::: "memory");
+}
+
+__device__ __forceinline__ void fence_proxy_async_global() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
 __device__ __forceinline__ void red_add_release_gpu(int* p, int v) {

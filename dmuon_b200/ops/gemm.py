@@ -396,7 +396,7 @@ def gemm(
     args.status = status_buffer(dev).data_ptr()
     args.max_ctas = int(max_ctas)
     args.two_cta = two_cta
-    rc = _fn()(ctypes.byref(args), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    rc = _fn()(ctypes.byref(args), ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(dev.index)))
     if rc != 0:
         raise RuntimeError(f"dmuon_gemm_sm100 failed with code {rc}")
     return out

@@ -58,6 +58,15 @@ class _CastArgs(ctypes.Structure):
     _fields_ = [
         ("src", _VP), ("dst", _VP), ("numel", _LL), ("slot", _IA), ("n", ctypes.c_int),
         ("src_dtype", ctypes.c_int), ("dst_dtype", ctypes.c_int), ("scale", ctypes.c_void_p),
+        ("sumsq", ctypes.c_void_p), ("norm_num", ctypes.c_float), ("norm_eps", ctypes.c_float),
+    ]
+
+
+class _RescaleArgs(ctypes.Structure):
+    _fields_ = [
+        ("sumsq", ctypes.c_void_p), ("k", ctypes.c_void_p), ("prescale", ctypes.c_void_p),
+        ("vec", ctypes.c_void_p), ("vec2", ctypes.c_void_p),
+        ("n", ctypes.c_int), ("fresh", ctypes.c_int), ("eps", ctypes.c_float),
     ]
 
 
@@ -67,6 +76,7 @@ def _lib():
     for name, typ in (
         ("dmuon_muon_prologue", _PrologueArgs),
         ("dmuon_norm_scales", _NormArgs),
+        ("dmuon_rescale", _RescaleArgs),
         ("dmuon_adamw", _AdamWArgs),
         ("dmuon_clip_sumsq", _ClipArgs),
         ("dmuon_clip_scale", _ClipArgs),
@@ -85,7 +95,8 @@ def launch_count() -> int:
 
 
 def _stream(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    # the raw handle: building a Stream object takes longer than the launch
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device.index))
 
 
 def _check(rc: int, what: str) -> None:
@@ -147,6 +158,19 @@ def norm_scales(sumsq: torch.Tensor, scale: torch.Tensor, scale2: torch.Tensor, 
     a.sumsq, a.scale, a.scale2 = sumsq.data_ptr(), scale.data_ptr(), scale2.data_ptr()
     a.n, a.eps = sumsq.numel(), float(eps)
     _check(_lib().dmuon_norm_scales(ctypes.byref(a), _stream(sumsq.device)), "dmuon_norm_scales")
+
+
+def rescale(
+    sumsq: torch.Tensor, k: torch.Tensor, prescale: torch.Tensor, vec: torch.Tensor, vec2: torch.Tensor,
+    fresh: bool, eps: float = 1e-7,
+) -> None:
+    """Correction factors of operands that are stored times ``prescale`` (see the
+    argument block in ``csrc/multi_tensor.cuh``); ``prescale`` is updated in place."""
+    a = _RescaleArgs()
+    a.sumsq, a.k, a.prescale = sumsq.data_ptr(), k.data_ptr(), prescale.data_ptr()
+    a.vec, a.vec2 = vec.data_ptr(), vec2.data_ptr()
+    a.n, a.fresh, a.eps = sumsq.numel(), int(bool(fresh)), float(eps)
+    _check(_lib().dmuon_rescale(ctypes.byref(a), _stream(sumsq.device)), "dmuon_rescale")
 
 
 def adamw(
@@ -225,8 +249,12 @@ def cast(
     dsts: Sequence[torch.Tensor],
     scale: Optional[torch.Tensor] = None,
     slots: Optional[Sequence[int]] = None,
+    sumsq: Optional[torch.Tensor] = None,
+    norm_num: float = 1.0,
+    norm_eps: float = 1e-7,
 ) -> None:
-    """``dst = cast(src * scale[slot])`` for many tensors in few launches."""
+    """``dst = cast(src * scale[slot])`` for many tensors in few launches; with
+    ``sumsq`` the scale is ``norm_num / (sqrt(sumsq[slot]) + norm_eps)``."""
     n = len(srcs)
     if n == 0:
         return
@@ -243,4 +271,6 @@ def cast(
         a.n = hi - lo
         a.src_dtype, a.dst_dtype = _DT[sd], _DT[dd]
         a.scale = scale.data_ptr() if scale is not None else None
+        a.sumsq = sumsq.data_ptr() if sumsq is not None else None
+        a.norm_num, a.norm_eps = float(norm_num), float(norm_eps)
         _check(_lib().dmuon_cast(ctypes.byref(a), _stream(dev)), "dmuon_cast")

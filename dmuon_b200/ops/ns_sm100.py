@@ -22,19 +22,25 @@ transposed copy is ever made):
     final         W = (1 - lr wd) W - lr * scale * Q X   written straight into
                   the fp32 master weights (and a bf16 publish copy)
 
-Symmetric products compute only the tiles that touch the lower triangle (the
-CTA-pair kernel, 256 x 256 tiles, whenever the shape fills it).
+Symmetric products compute only the tiles that touch the lower triangle (CTA
+pairs, 256 x 256 tiles, whenever the shapes fill them).  The products of one or
+more shape groups are issued as ONE launch of the product-chain kernel
+(:mod:`.chain`); one launch per product remains for gradients that are read from
+peers' memory, bf16 operands of the update, and outputs a plan does not take.
 Replaces the reference's per-matrix Python loop around SYRK / cuBLAS calls and
 its CUDA-graph cache (dmuon/optim/muon.py:1582-1747,
 dmuon/optim/newton_schulz.py:333-448, dmuon/optim/ns_graph.py:61-128).
 """
 from __future__ import annotations
 
+from dataclasses import dataclass
+from functools import cached_property, lru_cache
 from typing import Optional, Sequence
 
 import torch
 
 from . import build as _build
+from . import chain as CH
 from . import gemm as G
 from . import multi_tensor as MT
 
@@ -108,6 +114,7 @@ def release_workspaces() -> None:
     _workspaces.clear()
     _ptr_tables.clear()
     _prescales.clear()
+    CH.release()
 
 
 def max_batch(m0: int, n0: int, itemsize: int = 2) -> int:
@@ -170,10 +177,7 @@ class _XScale:
         self.vec, self.vec2, self.h = vec, vec2, float(h)
 
 
-def fp16_prescale(m0: int, n0: int) -> float:
-    import math
-
-    return float(2 ** round(math.log2(math.sqrt(min(m0, n0)))))
+fp16_prescale = CH.fp16_prescale
 
 
 def _iterate(ws: _Workspace, coefs, restarts, formulation: str, left: bool, xs: _XScale, segments=None):
@@ -246,6 +250,24 @@ def _run(ws: _Workspace, coefs, restarts, formulation: str, left: bool, xs: _XSc
     _apply(Q, X, left, **final_kw)
 
 
+def _chain_pays(specs: Sequence[CH.GroupSpec]) -> bool:
+    """Run these groups as one launch of the product-chain kernel?  Wherever a plan can
+    hold them: products only, one launch against one per product, B200: 105 / 231 us for
+    one matrix of 256 x 1024, 271 / 361 for 1152 x 4304, 309 / 668 for eight of
+    1024 x 1408, 1089 / 1237 for one of 3072 x 8192."""
+    return CH.possible(tuple(specs))
+
+
+def _aligned(tensors) -> bool:
+    return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
+
+
+@lru_cache(maxsize=4096)
+def _spec_of(L: int, m0: int, n0: int, cd: torch.dtype, formulation: str, coefs: tuple, restarts: tuple, h: float,
+             with_vec: bool) -> CH.GroupSpec:
+    return CH.GroupSpec(L, m0, n0, cd, formulation, coefs, restarts, h, with_vec)
+
+
 def _resolve_dtype(compute_dtype, formulation: str) -> torch.dtype:
     if compute_dtype in (torch.bfloat16, torch.float16):
         return compute_dtype
@@ -267,9 +289,26 @@ def newton_schulz_batched(
     assert X_in.dim() == 3 and X_in.is_cuda
     L, m0, n0 = X_in.shape
     cd = _resolve_dtype(compute_dtype, formulation)
-    ws = workspace(L, m0, n0, cd, X_in.device)
     left = m0 <= n0
     K = fp16_prescale(m0, n0) if (cd == torch.float16 and formulation == "gram") else 1.0
+    if out is None:
+        out = torch.empty(L, m0, n0, device=X_in.device, dtype=X_in.dtype)
+    if X_in.is_contiguous() and out.is_contiguous() and X_in.dtype in MT._DT and out.dtype in MT._DT \
+            and _aligned((out,)):
+        spec = _spec_of(L, m0, n0, cd, formulation, tuple(map(tuple, coefs)), tuple(restarts), 1.0 / K, False)
+        plan = CH.plan_for((spec,), X_in.device) if _chain_pays((spec,)) else None
+        if plan is not None:
+            mats, X = [X_in[i] for i in range(L)], plan.groups[0].X
+            res = out if formulation == "gram" or out.dtype == cd else torch.empty_like(out, dtype=cd)
+            with plan.lock:
+                plan.begin()
+                MT.clip_sumsq(mats, range(L), plan.sumsq)
+                MT.cast(mats, [X[i] for i in range(L)], slots=range(L), sumsq=plan.sumsq, norm_num=K, norm_eps=eps)
+                plan.run([dict(out=res)])
+            if res is not out:
+                out.copy_(res)
+            return out
+    ws = workspace(L, m0, n0, cd, X_in.device)
     if X_in.is_contiguous() and X_in.dtype in MT._DT:
         # one read for the norms, one read + one write for the normalised operand
         mats = [X_in[i] for i in range(L)]
@@ -286,8 +325,6 @@ def newton_schulz_batched(
         ws.scale.copy_(K / (sumsq.sqrt() + eps))
         ws.X.copy_(Xf * ws.scale.view(-1, 1, 1))
     xs = _XScale(h=1.0 / K)
-    if out is None:
-        out = torch.empty(L, m0, n0, device=X_in.device, dtype=X_in.dtype)
     kw: dict = {}
     if formulation == "direct":
         _run(ws, coefs, restarts, formulation, left, xs, kw)
@@ -366,6 +403,113 @@ def newton_schulz_single(G_in, coefs, restarts, eps, formulation, compute_dtype)
     if not X.is_contiguous():
         X = X.contiguous()
     return newton_schulz_batched(X, coefs, restarts, eps, formulation, compute_dtype).reshape(shape)
+
+
+@dataclass
+class UpdateJob:
+    """One shape group of a Muon step: the arguments of :func:`muon_update_batched`."""
+
+    grads: Optional[Sequence[torch.Tensor]]
+    moms: Sequence[torch.Tensor]
+    masters: Optional[Sequence[torch.Tensor]]
+    options: dict
+    publish: Optional[Sequence[Optional[torch.Tensor]]] = None
+    deltas: Optional[Sequence[torch.Tensor]] = None
+    publish_multicast: Optional[Sequence[int]] = None
+
+    @cached_property
+    def spec(self) -> CH.GroupSpec:
+        """Gram form, fp16 operands stored with last step's K / ||u|| (see
+        :func:`muon_update_batched`), the exact factor supplied per matrix."""
+        o = self.options
+        m0 = int(self.moms[0].shape[0])
+        return _spec_of(len(self.moms), m0, int(self.moms[0].numel() // m0), torch.float16, "gram",
+                        tuple(map(tuple, o["coefs"])), tuple(o["restarts"]), 1.0, True)
+
+    def chainable(self) -> bool:
+        o = self.options
+        return (o["formulation"] == "gram" and _resolve_dtype(o["compute_dtype"], "gram") == torch.float16
+                and SINGLE_PASS_FP16 and o.get("peer") is None and self.publish_multicast is None
+                and _aligned(self.masters or ()) and _aligned(self.deltas or ()) and _aligned(self.publish or ())
+                and _chain_pays((self.spec,)))
+
+
+def muon_update_groups(jobs: Sequence[UpdateJob], on_issued) -> None:
+    """:func:`muon_update_batched` for several shape groups.  Groups that are too small
+    to fill the GPU run side by side in shared launches of the product-chain kernel.
+    ``on_issued(i, wrote)`` is called as soon as the kernels of job ``i`` are issued
+    (``wrote`` as returned by :func:`muon_update_batched`), not after all jobs: callers
+    start communication there."""
+
+    def alone(i: int) -> None:
+        job = jobs[i]
+        on_issued(i, muon_update_batched(job.grads, job.moms, job.masters, deltas=job.deltas, publish=job.publish,
+                                         publish_multicast=job.publish_multicast, **job.options))
+
+    chunks: list[list[int]] = []
+    for i, job in enumerate(jobs):
+        if not job.moms or not job.chainable():
+            alone(i)
+        elif chunks and _chain_pays([*(jobs[k].spec for k in chunks[-1]), job.spec]):
+            chunks[-1].append(i)
+        else:
+            chunks.append([i])
+    for chunk in chunks:
+        part = [jobs[k] for k in chunk]
+        plan = CH.plan_for([j.spec for j in part], part[0].moms[0].device)
+        if plan is not None:
+            with plan.lock:
+                _muon_update_chain(plan, part)
+        for k in chunk:
+            if plan is None:
+                alone(k)
+            else:
+                job = jobs[k]
+                on_issued(k, job.deltas is None and _has_publish(job.publish))
+
+
+def _has_publish(publish) -> bool:
+    return publish is not None and all(p is not None for p in publish)
+
+
+def _muon_update_chain(plan: "CH.Plan", jobs: Sequence[UpdateJob]) -> None:
+    eps = 1e-7
+    moms = [m for j in jobs for m in j.moms]
+    owner_key = tuple(m.data_ptr() for m in moms)
+    pre = _prescales.get(owner_key)
+    fresh = pre is None
+    if fresh:
+        if len(_prescales) > 4096:
+            _prescales.clear()
+        pre = torch.empty_like(plan.vec)
+    operands = [grp.X[i] for grp in plan.groups for i in range(grp.spec.L)]
+    stage = [torch.empty(x.shape, dtype=torch.float32, device=x.device) for x in operands] if fresh else operands
+    slots = range(plan.n_matrices)
+    plan.begin()
+    first = 0
+    for j in jobs:
+        n, o = len(j.moms), j.options
+        MT.muon_prologue(j.grads, j.moms, stage[first : first + n], slots[first : first + n], plan.sumsq, o["mu"],
+                         o["nesterov"], o["gscale"], xscale=None if fresh else pre)
+        first += n
+    MT.rescale(plan.sumsq, plan.k, pre, plan.vec, plan.vec2, fresh, eps)
+    if fresh:
+        MT.cast(stage, operands, scale=pre, slots=slots)
+        _prescales[owner_key] = pre
+    finals = []
+    for j in jobs:
+        o = j.options
+        f = dict(alpha=-float(o["lr"]) * float(o["update_scale"]))
+        if j.deltas is not None:
+            f.update(out_tab=_ptr_table(j.deltas), out_dtype=j.deltas[0].dtype)
+        else:
+            tab = _ptr_table(j.masters)
+            f.update(out_tab=tab, c_tab=tab, out_dtype=j.masters[0].dtype,
+                     beta=1.0 - float(o["lr"]) * float(o["weight_decay"]))
+            if _has_publish(j.publish):
+                f.update(out2_tab=_ptr_table(j.publish))
+        finals.append(f)
+    plan.run(finals)
 
 
 def muon_update_batched(

@@ -850,6 +850,8 @@ class Muon(torch.optim.Optimizer):
             by_shape[key].append((dp, grad))
         coefs = self.ns.resolved_coefficients(self.ns_steps)
         restarts = self.ns.resolved_restarts()
+        jobs: list = []
+        after: list[tuple] = []         # (parameters, replicate the published copies) of each job
         for (rows, cols, gdt, _od, _md, is_tp, _has_pub), items in by_shape.items():
             cap = ns_sm100.max_batch(rows, cols)
             self._first_step_shape(rows, cols, len(items), "sm_100a kernels, batched by shape")
@@ -885,9 +887,8 @@ class Muon(torch.optim.Optimizer):
                             deltas.append(ex.delta_view(dp))
                         else:
                             deltas.append(torch.empty(dp.full_shape, dtype=torch.float32, device=self.device))
-                    ns_sm100.muon_update_batched(grads, moms, None, deltas=deltas, **common)
-                    for (dp, _), d in zip(chunk, deltas):
-                        dp._tp_full_delta = d
+                    jobs.append(ns_sm100.UpdateJob(grads, moms, None, common, deltas=deltas))
+                    after.append((chunk, False))
                 else:
                     masters = [dp._owned_data for dp, _ in chunk]
                     publish = [getattr(dp, "_publish_view", None) for dp, _ in chunk]
@@ -901,14 +902,24 @@ class Muon(torch.optim.Optimizer):
                             multicast = [rt.pub_mc + dp._arena_offset * esz for dp, _ in chunk]
                         else:
                             publish = [None] * len(chunk)       # published (cast + multicast) after the step
-                    wrote = ns_sm100.muon_update_batched(grads, moms, masters, publish=publish,
-                                                         publish_multicast=multicast, **common)
-                    if nvls and wrote and multicast is None:
-                        # the last product wrote the local slots: replicate them to all ranks on the
-                        # publish lane while the next batch is orthogonalised
-                        rt.multicast_publish_async([dp for dp, _ in chunk])
-                    for dp, _ in chunk:
-                        dp._publish_fresh = bool(wrote)
+                    jobs.append(ns_sm100.UpdateJob(grads, moms, masters, common, publish=publish,
+                                                   publish_multicast=multicast))
+                    after.append((chunk, nvls and multicast is None))
+
+        def issued(i: int, wrote: bool) -> None:
+            job, (chunk, replicate) = jobs[i], after[i]
+            if job.deltas is not None:
+                for (dp, _), d in zip(chunk, job.deltas):
+                    dp._tp_full_delta = d
+                return
+            if replicate and wrote:
+                # the last product wrote the local slots: replicate them to all ranks on the
+                # publish lane while the next batch is orthogonalised
+                rt.multicast_publish_async([dp for dp, _ in chunk])
+            for dp, _ in chunk:
+                dp._publish_fresh = bool(wrote)
+
+        ns_sm100.muon_update_groups(jobs, issued)
 
     # ------------------------------------------------------------------ AdamW
     def _adamw_state(self, key, like: torch.Tensor, dtype: torch.dtype) -> dict:

@@ -1,0 +1,124 @@
+"""The tile lists of the one-launch Newton-Schulz (``ops/chain.py``), interpreted on
+the CPU: dependencies, coverage and the numbers they produce."""
+import numpy as np
+import pytest
+import torch
+
+from dmuon_b200.ops import chain as CH
+from dmuon_b200.optim import newton_schulz as NS
+
+COEFS = tuple(map(tuple, NS.DEFAULT_COEFFICIENTS))
+
+
+def _spec(L, m0, n0, formulation="gram", restarts=(2,), coefs=COEFS, h=1.0, vec=False):
+    dt = torch.float16 if formulation == "gram" else torch.bfloat16
+    return CH.GroupSpec(L, m0, n0, dt, formulation, coefs, restarts if formulation == "gram" else (), h, vec)
+
+
+def _interpret(specs, bn, inputs):
+    """Run the list in order with fp64 arithmetic; every buffer starts as NaN, so a tile
+    that is read before it was written, or never written, shows in the result."""
+    ops, ent = CH.build_entries(specs, bn)
+    buf = []
+    for s, x in zip(specs, inputs):
+        names = ("R", "P") if s.formulation == "direct" else ("R", "R2", "RP", "P", "Qa", "Qb")
+        d = {n: np.full((s.L, s.m, s.m), np.nan) for n in names}
+        d["X"], d["X2"] = x.copy(), np.full_like(x, np.nan)
+        d["final"] = np.full_like(x, np.nan)
+        d["parts"] = None
+        buf.append(d)
+    first = np.cumsum([0] + [s.L for s in specs])
+    done = np.zeros(first[-1], dtype=np.int64)
+    # what has to be finished before a product may start, per matrix: everything up to `after`
+    finished_by_op = [{} for _ in range(first[-1])]
+
+    def tile(s, d, pr, ns, per, is_sum, b, split, mirror, rows, cols, r0, r1, c0, c1):
+        assert r0 < rows and c0 < cols
+        if is_sum:
+            v = d["parts"][b].sum(0)[r0:r1, c0:c1]
+        else:
+            A = d[pr.A][b].T if pr.a_mn else d[pr.A][b]
+            B = d[pr.B][b].T if pr.b_mn else d[pr.B][b]
+            lo, hi = (split * per * 64, min(A.shape[1], (split + 1) * per * 64)) if per else (0, A.shape[1])
+            assert lo < hi
+            v = A[r0:r1, lo:hi] @ B[c0:c1, lo:hi].T
+        if ns > 1 and not is_sum:
+            if d["parts"] is None or d["parts"].shape[1] != ns:
+                d["parts"] = np.full((s.L, ns, rows, cols), np.nan)
+            d["parts"][b, split, r0:r1, c0:c1] = v
+        else:
+            v = pr.alpha * v
+            if pr.C is not None:
+                v = v + pr.beta * d[pr.C][b][r0:r1, c0:c1]
+            v = v + pr.diag * np.eye(rows, cols)[r0:r1, c0:c1]
+            d[pr.out][b, r0:r1, c0:c1] = v
+            if mirror:
+                d[pr.out][b, c0:c1, r0:r1] = v.T
+
+    for x, y, z, w in ent.astype(np.int64):
+        op, mirror, split = x & 0xFF, (x >> 8) & 1, (x >> 16) & 0x7FFF
+        mt, nt, b, ctr = y & 0xFFFF, (y >> 16) & 0xFFFF, z & 0xFFFF, (z >> 16) & 0xFFFF
+        g, pr, ns, per, is_sum = ops[op]
+        s, d = specs[g], buf[g]
+        assert ctr == first[g] + b and done[ctr] >= w
+        assert x >= 0
+        rows = s.m if pr.symmetric else s.m0
+        cols = s.m if pr.symmetric else s.n0
+        tn, tm = CH._SUM_COLS if is_sum else bn, CH.tile_rows(bn)
+        r0, r1, c0, c1 = mt * tm, min(rows, mt * tm + tm), nt * tn, min(cols, nt * tn + tn)
+        tile(s, d, pr, ns, per, is_sum, b, split, mirror, rows, cols, r0, r1, c0, c1)
+        done[ctr] += CH.WARPS_PER_TILE * (2 if bn == CH.PAIR else 1)
+        finished_by_op[ctr][op] = done[ctr]
+    # a count in the list stands for whole products: w equals the count after `after` finished
+    ends = {}
+    for i, (g, pr, ns, per, is_sum) in enumerate(ops):
+        ends[g] = ends.get(g, []) + [(i, ns > 1 and not is_sum)]
+    for x, y, z, w in ent.astype(np.int64):
+        op, ctr = x & 0xFF, (z >> 16) & 0xFFFF
+        assert w == 0 or w in set(finished_by_op[ctr].values())
+        assert w == 0 or max(o for o, c in finished_by_op[ctr].items() if c <= w) < op
+    return [d["final"] for d in buf]
+
+
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("shapes,formulation", [
+    ([(1, 64, 96)], "gram"), ([(2, 128, 128)], "gram"), ([(1, 136, 1040)], "gram"), ([(1, 2056, 72)], "gram"),
+    ([(3, 264, 200)], "direct"), ([(1, 72, 1544)], "direct"),
+    ([(2, 256, 128), (1, 128, 328), (2, 72, 64)], "gram"), ([(2, 1096, 600)], "gram"), ([(30, 264, 64)], "gram"),
+])
+def test_tile_list_computes_the_iteration(shapes, formulation, bn):
+    rng = np.random.default_rng(0)
+    specs = [_spec(L, m0, n0, formulation) for L, m0, n0 in shapes]
+    xs = []
+    for s in specs:
+        x = rng.standard_normal((s.L, s.m0, s.n0))
+        xs.append(x / np.linalg.norm(x, axis=(1, 2), keepdims=True))
+    for s, x, out in zip(specs, xs, _interpret(specs, bn, xs)):
+        for b in range(s.L):
+            want = NS.direct_newton_schulz(torch.from_numpy(x[b]).double(), coefficients=s.coefs, eps=0.0,
+                                           compute_dtype=torch.float64).numpy()
+            # fp32 normalisation in the oracle, fp64 products on both sides
+            assert np.abs(out[b] - want).max() < 1e-4 * np.abs(want).max()
+
+
+def test_restart_variants_and_scale_factors():
+    rng = np.random.default_rng(1)
+    for restarts in ((), (1,), (2, 4), (0, 3)):
+        s = _spec(1, 64, 136, restarts=restarts, h=0.25)
+        x = rng.standard_normal((1, 64, 136))
+        x /= np.linalg.norm(x)
+        out = _interpret([s], 64, [x * 4.0])[0]
+        want = NS.direct_newton_schulz(torch.from_numpy(x[0]).double(), coefficients=COEFS, eps=0.0,
+                                       compute_dtype=torch.float64).numpy()
+        assert np.abs(out[0] - want).max() < 1e-4 * np.abs(want).max()
+
+
+def test_limits_of_a_plan():
+    assert CH.fits([_spec(1, 128, 128)])
+    assert not CH.fits([_spec(1, 128, 100)])                       # pitches are multiples of eight
+    assert not CH.fits([_spec(1, 128, 128, coefs=COEFS * 20)])     # too many products
+    assert not CH.fits([_spec(1, 128, 128)] * 17)
+    for L, m, n in ((1, 128, 14336), (1, 1152, 4304), (8, 256, 256), (1, 128, 128)):
+        spl, per = CH.gram_splits(_spec(L, m, n), 128, CH.sym_tiles([_spec(L, m, n)], 128))
+        kb = -(-n // 64)
+        assert spl * per >= kb and (spl - 1) * per < kb and 1 <= spl <= 16

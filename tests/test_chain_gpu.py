@@ -1,0 +1,118 @@
+"""One-launch Newton-Schulz (``csrc/chain_sm100.cu``) against 64-bit math (needs a B200)."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev():
+    return torch.device("cuda", 0)
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+@pytest.mark.parametrize("formulation", ["gram", "direct"])
+@pytest.mark.parametrize("L,m0,n0,dt", [
+    (1, 8, 64, torch.float32),            # far below one tile
+    (1, 128, 128, torch.bfloat16),        # exactly one row of tiles
+    (2, 136, 1040, torch.float32),        # remainders in every dimension, Gram split over K
+    (1, 1152, 4304, torch.bfloat16),      # no multiple of a tile, full-width tiles, split
+    (1, 4096, 200, torch.float32),        # tall: MN-major operands, split
+    (1, 520, 520, torch.float32),         # full-width and half-width remainders of the mirror
+    (5, 256, 256, torch.bfloat16),        # batch, several tickets per CTA
+    (12, 1032, 1160, torch.bfloat16),     # CTA pairs, remainders in every dimension
+    (75, 264, 128, torch.float32),        # CTA pairs, MN-major operands, K below one trip of the stage ring
+])
+def test_chain_matches_64_bit_iteration(L, m0, n0, dt, formulation, monkeypatch):
+    from dmuon_b200.ops import chain as CH
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+
+    torch.manual_seed(m0 + n0)
+    coefs = list(NS.DEFAULT_COEFFICIENTS)
+    restarts = [2] if formulation == "gram" else []
+    X = (torch.randn(L, m0, n0, device=_dev()) * 1e-3).to(dt)
+    for _ in range(3):                    # the kernel clears its counters for the next call
+        out = ns_sm100.newton_schulz_batched(X, coefs, restarts, 1e-7, formulation)
+    torch.cuda.synchronize()
+    G.check_status(_dev())
+    assert any(k[0][0][0].m0 == m0 and k[0][0][0].formulation == formulation for k in CH._plans)
+    # the same products as one launch each: same operand roundings, 32-bit sums in the same order (another one where
+    # a Gram product is split over K), so the two differ by what one changed rounding grows to in five steps
+    monkeypatch.setattr(ns_sm100, "_chain_pays", lambda specs: False)
+    alone = ns_sm100.newton_schulz_batched(X, coefs, restarts, 1e-7, formulation)
+    torch.cuda.synchronize()
+    G.check_status(_dev())
+    for i in range(L):
+        exact = NS.direct_newton_schulz(X[i].double(), coefficients=coefs, compute_dtype=torch.float64)
+        limit = 1.25 * _rel(alone[i], exact) + (2e-3 if formulation == "gram" else 8e-3)
+        assert _rel(out[i], exact) < limit
+
+
+def test_grouped_update_of_several_shapes_matches_fp32_math():
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+
+    dev = _dev()
+    torch.manual_seed(4)
+    shapes = [(3, 256, 256), (2, 1024, 256), (2, 136, 512)]
+    coefs, restarts, lr, wd, mu = list(NS.DEFAULT_COEFFICIENTS), [2], 0.02, 0.1, 0.9
+    moms = [[torch.zeros(m, n, device=dev) for _ in range(L)] for L, m, n in shapes]
+    masters = [[torch.randn(m, n, device=dev) * 0.02 for _ in range(L)] for L, m, n in shapes]
+    pubs = [[torch.zeros(m, n, device=dev, dtype=torch.bfloat16) for _ in range(L)] for L, m, n in shapes]
+    for step, mag in enumerate([1e-3, 5e-3, 2.5e-4]):
+        grads = [[(torch.randn(m, n, device=dev) * mag).bfloat16() for _ in range(L)] for L, m, n in shapes]
+        m_prev = [[x.clone() for x in g] for g in moms]
+        w_prev = [[x.clone() for x in g] for g in masters]
+        jobs = []
+        for g, (L, m, n) in enumerate(shapes):
+            options = dict(mu=mu, nesterov=True, coefs=coefs, restarts=restarts, formulation="gram", lr=lr,
+                           weight_decay=wd, update_scale=0.2 * math.sqrt(max(m, n)), compute_dtype=None, gscale=None,
+                           peer=None)
+            jobs.append(ns_sm100.UpdateJob(grads[g], moms[g], masters[g], options, publish=pubs[g] if g else None))
+        issued = {}
+        ns_sm100.muon_update_groups(jobs, issued.__setitem__)
+        torch.cuda.synchronize()
+        G.check_status(dev)
+        assert issued == {0: False, 1: True, 2: True}
+        for g, (L, m, n) in enumerate(shapes):
+            scale = 0.2 * math.sqrt(max(m, n))
+            for i in range(L):
+                buf = mu * m_prev[g][i] + grads[g][i].float()
+                u = grads[g][i].float() + mu * buf
+                o = NS.gram_newton_schulz(u, coefficients=coefs, restart_iterations=restarts, deterministic=True,
+                                          compute_dtype=torch.float32)
+                ref = w_prev[g][i] * (1 - lr * wd) - lr * scale * o
+                assert torch.allclose(moms[g][i], buf, atol=1e-6), (step, g)
+                assert (masters[g][i] - ref).abs().max().item() < 0.1 * lr * scale, (step, g)
+                if g:
+                    assert torch.equal(pubs[g][i], masters[g][i].bfloat16())
+
+
+def test_chain_on_two_streams_at_once():
+    """Plans are per stream: calls of one shape on two streams do not share buffers."""
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+
+    coefs, dev = list(NS.DEFAULT_COEFFICIENTS), _dev()
+    torch.manual_seed(5)
+    X = [torch.randn(1, 256, 640, device=dev) for _ in range(2)]
+    want = [ns_sm100.newton_schulz_batched(x, coefs, [2]) for x in X]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream(dev) for _ in X], []
+    for _ in range(8):
+        for x, s in zip(X, streams):
+            with torch.cuda.stream(s):
+                got.append(ns_sm100.newton_schulz_batched(x, coefs, [2]))
+    torch.cuda.synchronize()
+    G.check_status(dev)
+    for k, o in enumerate(got):
+        # the norm is an atomic sum: its last bit, amplified by five fp16 steps
+        assert _rel(o, want[k % 2].double()) < 2e-2
