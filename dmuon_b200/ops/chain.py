@@ -30,6 +30,7 @@ from . import gemm as G
 MAX_OPS = 76
 MAX_GROUPS = 16
 SMS = 148
+PAIRS = SMS // 2
 _KB = 64                      # inner elements per pipeline stage
 _SUM_COLS = 64                # columns of one entry of a sum of partial products
 WARPS_PER_TILE = 8            # epilogue warps per CTA: each reports a finished tile
@@ -66,8 +67,8 @@ class _Map(ctypes.Structure):
 class _Args(ctypes.Structure):
     _fields_ = [
         ("ops", _VP), ("maps", _VP), ("tab", _VP), ("counters", _VP), ("status", _VP),
-        ("n_ops", _I), ("n_maps", _I), ("total", _I), ("n_counters", _I), ("n_final", _I), ("bn", _I),
-        ("max_ctas", _I), ("pad_", _I),
+        ("n_ops", _I), ("n_maps", _I), ("total", _I), ("n_counters", _I), ("n_final", _I),
+        ("max_ctas", _I), ("bn", _I), ("wide", _I),
         ("fin", _Final * MAX_GROUPS),
     ]
 
@@ -215,9 +216,14 @@ def _tiles(m: int, n: int, bn: int, symmetric: bool) -> np.ndarray:
     return np.asarray(t, dtype=np.int64).reshape(-1, 3)
 
 
+@lru_cache(maxsize=4096)
+def sym_tile_count(m: int, bn: int) -> int:
+    return len(G.symmetric_tiles(m, bn, tile_rows(bn)))
+
+
 def sym_tiles(specs: Sequence[GroupSpec], bn: int) -> int:
     """Tiles of one symmetric product of every group."""
-    return sum(s.L * len(G.symmetric_tiles(s.m, bn, tile_rows(bn))) for s in specs)
+    return sum(s.L * sym_tile_count(s.m, bn) for s in specs)
 
 
 def fits(specs: Sequence[GroupSpec]) -> bool:
@@ -231,14 +237,62 @@ def fits(specs: Sequence[GroupSpec]) -> bool:
     return sum(len(p) + split * sum(q.symmetric and q.A in ("X", "X2") for q in p) for p in map(_products_of, specs)) <= MAX_OPS
 
 
+#: tile width -> (CTAs or pairs that work at once; microseconds per k-block of a tile when few of them work; when
+#: all do; microseconds from the first load of a product to the first load of the next beyond its k-blocks)
+_COST = {64: (SMS, 0.31, 0.40, 4.2), 128: (SMS, 0.41, 0.52, 5.0), PAIR: (PAIRS, 0.42, 0.46, 7.0)}
+
+
+def estimate_us(specs: Sequence[GroupSpec], bn: int) -> float:
+    """Time of a chain with this tile width: product by product, the k-blocks of its longest
+    round plus the way from one product to the next.  An SM is fed about 80 bytes per
+    nanosecond, so a k-block costs what its operands weigh (24, 32 and 32 KB per SM here), a
+    little more when all SMs pull.  Measured / estimated on a B200: 256 x 256 97 / 98, 1024 x
+    1024 in 64-wide tiles 222 / 180, 1536 x 1536 in 128-wide ones 278 / 295, 4096 x 4096 on
+    pairs 1301 / 1304, 4096 x 14336 2114 / 2128."""
+    units, alone, busy, step = _COST[bn]
+    tiles_all = sym_tiles(specs, bn)
+    matrices = sum(s.L for s in specs)
+    per_group = [_products_of(s) for s in specs]
+    total = 0.0
+    for i in range(max(len(p) for p in per_group)):
+        tiles = work = longest = 0
+        total += step
+        for s, products in zip(specs, per_group):
+            if i >= len(products):
+                continue
+            pr = products[i]
+            is_gram = pr.symmetric and pr.A in ("X", "X2")
+            splits, per = gram_splits(s, bn, tiles_all) if is_gram else (1, 0)
+            kb = per if splits > 1 else -(-(s.n if is_gram else s.m) // _KB)
+            if splits > 1:
+                total += step
+            n = splits * s.L * (sym_tile_count(s.m, bn) if pr.symmetric else
+                                -(-s.m0 // tile_rows(bn)) * -(-s.n0 // bn))
+            tiles, work, longest = tiles + n, work + n * kb, max(longest, kb)
+        # one or two matrices: whole rounds; more: tiles of other matrices fill the last one
+        rounds = max(longest, work / units) if matrices > 2 else -(-tiles // units) * longest
+        total += rounds * (alone + (busy - alone) * min(1.0, tiles / units))
+    return total
+
+
+@lru_cache(maxsize=4096)
+def _best_bn(specs: tuple) -> int:
+    return min(_COST, key=lambda bn: estimate_us(specs, bn))
+
+
 def choose_bn(specs: Sequence[GroupSpec]) -> int:
-    """CTA pairs once a symmetric product of all groups has a 256 x 256 tile for each
-    of them.  Below that, half-width tiles while 128-wide ones leave half of the SMs
-    without work: an SM is fed 64 bytes per clock, so more SMs with less each finish
-    sooner."""
-    if sym_tiles(specs, PAIR) * 2 >= SMS:
-        return PAIR
-    return 64 if sym_tiles(specs, 128) * 2 <= SMS else 128
+    """The tile width with the lowest estimate.  64-wide tiles where products are small (more
+    SMs with less each), CTA pairs where they fill the GPU or are long."""
+    return _best_bn(tuple(specs))
+
+
+def choose_wide(specs: Sequence[GroupSpec], bn: int) -> bool:
+    """Two tiles side by side per entry?  Only in lists with several rounds of tiles in every
+    product: an entry takes twice as long, so the last round of a product costs twice as much.
+    Measured (ms, single / two): four 14336 x 4096 (544 tiles a symmetric product) 9.89 / 8.91,
+    eight 4096 x 4096 (1088) 10.24 / 10.11, four 3072 x 8192 (312) 3.44 / 3.57, one
+    4096 x 14336 (136) 2.39 / 2.49."""
+    return bn == PAIR and sym_tiles(specs, PAIR) >= 3 * SMS
 
 
 def gram_splits(spec: GroupSpec, bn: int, tiles_all: int) -> tuple[int, int]:
@@ -300,6 +354,32 @@ class Group:
         self.partials: Optional[torch.Tensor] = self.buffers.get("partials")
 
 
+def _two_wide(e: np.ndarray) -> np.ndarray:
+    """Entries of 256 x 256 tiles joined into pairs that lie side by side (they share
+    their A rows, see the kernel): bit 9 = there is a second half, bit 10 = its mirror
+    flag.  What is left of a last round of single tiles stays single, at the end: a
+    round of wide tiles takes twice as long."""
+    left = len(e) % SMS
+    wide = len(e) - (left if left <= PAIRS else 0)
+    if wide == 0:
+        return e
+    row = (e[:wide, 0] & 0xFF) | ((e[:wide, 1] & 0xFFFF) << 8) | (e[:wide, 2] << 24)     # product, row of tiles, matrix
+    col = e[:wide, 1] >> 16
+    order = np.lexsort((col, row))
+    r, c = row[order], col[order]
+    at = np.arange(wide)
+    starts = np.r_[True, (r[1:] != r[:-1]) | (c[1:] != c[:-1] + 1)]              # runs of neighbours
+    inside = at - np.maximum.accumulate(np.where(starts, at, 0))
+    last = np.r_[starts[1:], True]
+    first = (inside % 2 == 0) & ~last
+    second = np.r_[False, first[:-1]]
+    joined = e[order[first]].copy()
+    joined[:, 0] |= (1 << 9) | (((e[order[second], 0] >> 8) & 1) << 10)
+    joined = joined[np.argsort(order[first], kind="stable")]                     # the list's own order: L2 locality
+    single = np.sort(np.r_[order[~first & ~second], np.arange(wide, len(e))])
+    return np.concatenate([joined, e[single]])
+
+
 def build_entries(specs: Sequence[GroupSpec], bn: int):
     """Products and tile list of a plan, without touching a device.
 
@@ -324,10 +404,12 @@ def build_entries(specs: Sequence[GroupSpec], bn: int):
         e[:, 1] = t[:, 0] | (t[:, 1] << 16)
         e[:, 2] = b | ((first_matrix[g] + b) << 16)
         e[:, 3] = want
-        chunks.append(e)
+        level.append(e)
         total[g] += len(tiles) * WARPS_PER_TILE * (2 if bn == PAIR else 1)
 
+    wide = choose_wide(specs, bn)
     for i in range(max(len(p) for p in per_group)):
+        level: list[np.ndarray] = []
         for g, s in enumerate(specs):
             if i >= len(per_group[g]):
                 continue
@@ -350,6 +432,8 @@ def build_entries(specs: Sequence[GroupSpec], bn: int):
                 ops.append((g, pr, 1, 0, False))
                 emit(g, len(ops) - 1, tiles, want)
             upto[g].append(total[g])
+        entries = np.concatenate(level)
+        chunks.append(_two_wide(entries) if wide else entries)
     entries = np.concatenate(chunks) if chunks else np.zeros((0, 4), dtype=np.int64)
     # the packing holds 31 bits per word; the sign bit of the first word marks the end of the list
     return ops, (entries & 0xFFFFFFFF).astype(np.uint32).view(np.int32)
@@ -362,6 +446,7 @@ class Plan:
         self.bn = choose_bn(self.specs)
         self.arena = arena
         self.lock = arena.lock
+        self.wide = choose_wide(self.specs, self.bn)
         tiles = sym_tiles(self.specs, self.bn)
         arena.used = 0
         self.groups = [Group(s, gram_splits(s, self.bn, tiles)[0], arena) for s in self.specs]
@@ -389,6 +474,7 @@ class Plan:
         a.counters, a.status = self.counters.data_ptr(), G.status_buffer(device).data_ptr()
         a.n_ops, a.n_maps, a.total = self.n_ops, self.n_maps, self.total
         a.n_counters, a.n_final, a.bn = self.counters.numel(), len(self.specs), self.bn
+        a.wide = int(self.wide)
         self._args = a
 
     def _encode(self, ops) -> None:

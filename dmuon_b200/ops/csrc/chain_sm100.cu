@@ -222,10 +222,6 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(const __grid_co
         ++cnt;
         if (e.x < 0) break;
         const OpS& op = ops[entry_op(e)];
-        if (op.map_a < 0) {
-          t = atomicAdd(ticket, 1);
-          continue;
-        }
         if (e.w > 0) {
           if (!wait_count(done + entry_ctr(e), e.w, abort_flag)) {
             fail_code = kStatusTimeoutPeerFlag;
@@ -237,6 +233,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(const __grid_co
         // Drawn before the wait, a CTA would sit on two tiles of a product while others idle
         // (1024 x 1024: 252 us for the chain).
         t = atomicAdd(ticket, 1);
+        if (op.map_a < 0) continue;        // a sum: the epilogue warps do all of it
         const CUtensorMap* tmA = p.maps + op.map_a;
         const CUtensorMap* tmB = p.maps + op.map_b;
         const int m0 = entry_m(e) * BM, n0 = entry_n(e) * BN, b = entry_b(e);
@@ -445,41 +442,63 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(const __grid_co
   }
 }
 
-// ---- CTA pairs (cta_group::2): 256 x 256 tiles -------------------------------------
+// ---- CTA pairs (cta_group::2) --------------------------------------------------------
 //
-// Same list, same counters; an entry is a 256 x 256 tile that two CTAs of a cluster
+// Same list, same counters; an entry is a tile of 256 rows that two CTAs of a cluster
 // share (128 rows each, MMAs issued by the leader).  The leader's producer draws the
-// tickets and writes every entry into both CTAs' rings.  For lists whose products
-// fill the GPU: per k-block a CTA pulls 32 KB from L2 for 512 clocks of MMA.  What it
-// gains over one launch per product is the tail of every product: tiles of other
-// matrices fill it.  No split over K: there are tiles enough.
-constexpr int kPairStages = 6;
-constexpr int kPairABytes = BM * BK * 2;            // 128 rows per CTA
-constexpr int kPairBBytes = 128 * BK * 2;           // 128 of the 256 columns per CTA
-constexpr int kPairStageBytes = kPairABytes + kPairBBytes;
+// tickets and writes every entry into both CTAs' rings.  For lists whose products fill
+// the GPU; no split over K, there are tiles enough.
+//
+// What bounds it is the L2 -> SM stream, which delivers about 80 bytes per nanosecond to
+// an SM (302 ns per 24 KB k-block on an otherwise idle GPU with every stage free): with
+// 256 columns a CTA pulls 32 KB per k-block for 512 clocks of MMA.
+//
+// WIDE: an entry is one or two such tiles side by side.  Two share their A rows, 48 KB
+// for 1024 clocks.  Both fill the tensor memory, so the next entry cannot use a second
+// accumulator set; instead the halves run out of step by the depth of the stage ring: the
+// last k-blocks of an entry are done for half 0 first, then for half 1, and so are the
+// first ones of the next entry.  While one half runs, the epilogue drains the other.
+// Pays for long lists only (choose_wide in ops/chain.py has the line and the figures).
+template <bool WIDE>
+struct PairCfg {
+  static constexpr int kStages = WIDE ? 4 : 6;
+  static constexpr int kABytes = BM * BK * 2;            // 128 rows per CTA
+  static constexpr int kBBytes = 128 * BK * 2;           // 128 of the 256 columns of a half per CTA
+  static constexpr int kHalves = WIDE ? 2 : 1;
+  static constexpr int kStageBytes = kABytes + kHalves * kBBytes;
+};
 constexpr int kPairBN = 256;
+template <bool WIDE>
 constexpr int pair_smem_bytes(int n_ops) {
-  return kPairStages * kPairStageBytes + kBarBytes + kStageBytesAll + n_ops * static_cast<int>(sizeof(OpS)) + 1024;
+  return PairCfg<WIDE>::kStages * PairCfg<WIDE>::kStageBytes + kBarBytes + kStageBytesAll +
+         n_ops * static_cast<int>(sizeof(OpS)) + 1024;
 }
 
+// flags of a wide entry: bit 8 / 10 = mirror half 0 / 1, bit 9 = there is a half 1
+template <bool WIDE>
+__device__ __forceinline__ int entry_halves(const int4& e) { return WIDE ? 1 + ((e.x >> 9) & 1) : 1; }
+__device__ __forceinline__ bool entry_mirror_half(const int4& e, int h) { return (e.x >> (8 + 2 * h)) & 1; }
+
+template <bool WIDE>
 __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __grid_constant__ ChainParams p) {
-  constexpr int S = kPairStages;
+  using C = PairCfg<WIDE>;
+  constexpr int S = C::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
-  uint8_t* sB = smem + S * kPairABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * kPairStageBytes);
+  uint8_t* sB = smem + S * C::kABytes;              // per stage: half 0, then half 1
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * C::kStageBytes);
   const uint32_t full0 = smem_u32(bars);
   const uint32_t empty0 = smem_u32(bars + S);
   const uint32_t tfull0 = smem_u32(bars + 2 * S);
   const uint32_t tempty0 = smem_u32(bars + 2 * S + 2);
   const uint32_t rfull0 = smem_u32(bars + 2 * S + 4);
   const uint32_t rempty0 = smem_u32(bars + 2 * S + 4 + kRing);
-  int4* ring = reinterpret_cast<int4*>(bars + 2 * S + 4 + 2 * kRing);
+  int4* ring = reinterpret_cast<int4*>(bars + 2 * S + 4 + 2 * kRing);     // an even number of 8-byte words in
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring + kRing);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint8_t* staging = smem + S * kPairStageBytes + kBarBytes;
+  uint8_t* staging = smem + S * C::kStageBytes + kBarBytes;
   OpS* ops = reinterpret_cast<OpS*>(staging + kStageBytesAll);
 
   const int warp = threadIdx.x >> 5;
@@ -564,21 +583,22 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
         if (leader) t = atomicAdd(ticket, 1);    // once this tile can run, see above
         const CUtensorMap* tmA = p.maps + op.map_a;
         const CUtensorMap* tmB = p.maps + op.map_b;
+        const int halves = entry_halves<WIDE>(e);
         const int m0 = entry_m(e) * 256 + 128 * static_cast<int>(rank);
         const int n0 = entry_n(e) * kPairBN + 128 * static_cast<int>(rank);
         const int b = entry_b(e);
         const int a_mn = op.k.a_mn_major, b_mn = op.k.b_mn_major;
         const int num_kb = (op.k.K + BK - 1) / BK;
+        const uint32_t bytes = 2 * (C::kABytes + halves * C::kBBytes);    // of both CTAs
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_bounded(empty0 + 8 * stage, phase ^ 1u, abort_flag)) {
             ok = false;
             fail_code = kStatusTimeoutProducer;
             break;
           }
-          if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * kPairStageBytes);
+          if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, bytes);
           const uint32_t fb = (full0 + 8 * stage) & 0xFEFFFFFFu;     // the leader's barrier
-          const uint32_t a_dst = smem_u32(sA + stage * kPairABytes);
-          const uint32_t b_dst = smem_u32(sB + stage * kPairBBytes);
+          const uint32_t a_dst = smem_u32(sA + stage * C::kABytes);
           if (!a_mn) {
             tma_load_3d_pair(a_dst, tmA, fb, kb * BK, m0, b);
           } else {
@@ -586,12 +606,16 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
             for (int mb = 0; mb < 2; ++mb)
               tma_load_3d_pair(a_dst + mb * kBlockBytes, tmA, fb, m0 + 64 * mb, kb * BK, b);
           }
-          if (!b_mn) {
-            tma_load_3d_pair(b_dst, tmB, fb, kb * BK, n0, b);
-          } else {
+          for (int h = 0; h < halves; ++h) {
+            const uint32_t b_dst = smem_u32(sB + (C::kHalves * stage + h) * C::kBBytes);
+            const int n = n0 + h * kPairBN;
+            if (!b_mn) {
+              tma_load_3d_pair(b_dst, tmB, fb, kb * BK, n, b);
+            } else {
 #pragma unroll
-            for (int nb = 0; nb < 2; ++nb)
-              tma_load_3d_pair(b_dst + nb * kBlockBytes, tmB, fb, n0 + 64 * nb, kb * BK, b);
+              for (int nb = 0; nb < 2; ++nb)
+                tma_load_3d_pair(b_dst + nb * kBlockBytes, tmB, fb, n + 64 * nb, kb * BK, b);
+            }
           }
           if (++stage == S) {
             stage = 0;
@@ -603,12 +627,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
   } else if (warp == 1) {
     if (lane == 0 && leader) {
       // ---------------- MMA issuer (leader only) ----------------
-      int stage = 0;
-      uint32_t phase = 0;
+      uint32_t it = 0;                     // k-blocks consumed so far: stage it % S, trip it / S
       int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (uint32_t cnt = 0; ok; ++cnt) {
+      uint32_t acc_phase = 0;              // one bit per accumulator
+      for (uint32_t cnt = 0;; ++cnt) {
         const uint32_t slot = cnt % kRing;
         if (!mbar_wait_bounded(rfull0 + 8 * slot, (cnt / kRing) & 1u, abort_flag)) {
           fail_code = kStatusTimeoutMma;
@@ -618,24 +640,28 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
         mbar_arrive(rempty0 + 8 * slot);
         if (e.x < 0) break;
         const OpS& op = ops[entry_op(e)];
-        if (!mbar_wait_bounded(tempty0 + 8 * acc, acc_phase ^ 1u, abort_flag)) {
-          fail_code = kStatusTimeoutMma;
-          break;
-        }
-        tc_fence_after_sync();
         const int a_mn = op.k.a_mn_major, b_mn = op.k.b_mn_major;
         const uint32_t idesc = make_idesc_f16(256, kPairBN, op.k.ab_fp16 != 0, a_mn != 0, b_mn != 0);
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kPairBN);
         const int num_kb = (op.k.K + BK - 1) / BK;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(full0 + 8 * stage, phase, abort_flag)) {
-            ok = false;
-            fail_code = kStatusTimeoutMma;
-            break;
-          }
+        const int halves = entry_halves<WIDE>(e);
+
+        auto wait_acc = [&](int a) -> bool {          // accumulator `a` has been drained
+          const bool r = mbar_wait_bounded(tempty0 + 8 * a, ((acc_phase >> a) & 1u) ^ 1u, abort_flag);
+          acc_phase ^= 1u << a;
           tc_fence_after_sync();
-          const uint32_t a_base = smem_u32(sA + stage * kPairABytes);
-          const uint32_t b_base = smem_u32(sB + stage * kPairBBytes);
+          return r;
+        };
+        auto wait_full = [&](int kb) -> bool {
+          const uint32_t i = it + kb;
+          const bool r = mbar_wait_bounded(full0 + 8 * (i % S), (i / S) & 1u, abort_flag);
+          tc_fence_after_sync();
+          return r;
+        };
+        auto mma = [&](int a, int h, int kb) {        // one k-block of half h into accumulator a
+          const uint32_t st = (it + kb) % S;
+          const uint32_t a_base = smem_u32(sA + st * C::kABytes);
+          const uint32_t b_base = smem_u32(sB + (C::kHalves * st + h) * C::kBBytes);
+          const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(a * kPairBN);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t adesc = a_mn ? make_smem_desc_sw128(a_base + k * 2048, kBlockBytes, 1024)
@@ -644,28 +670,70 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
                                         : make_smem_desc_sw128(b_base + k * 32, 16, 1024);
             umma_f16_ss_pair(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
           }
-          umma_commit_pair(mapa_shared(empty0 + 8 * stage, 0));
-          umma_commit_pair(mapa_shared(empty0 + 8 * stage, 1));
-          if (++stage == S) {
-            stage = 0;
-            phase ^= 1u;
+        };
+        auto commit = [&](uint32_t bar) {             // the MMAs so far, in both CTAs
+          umma_commit_pair(mapa_shared(bar, 0));
+          umma_commit_pair(mapa_shared(bar, 1));
+        };
+
+        bool ok = wait_acc(acc);
+        if (halves == 1) {
+          for (int kb = 0; ok && kb < num_kb; ++kb) {
+            ok = wait_full(kb);
+            if (!ok) break;
+            mma(acc, 0, kb);
+            commit(empty0 + 8 * ((it + kb) % S));
           }
+          if (ok) commit(tfull0 + 8 * acc);
+          acc ^= 1;
+        } else {
+          // k-blocks [0, head) and [tail, num_kb) half by half, those between together
+          const int head = min(S, num_kb);
+          const int tail = max(head, num_kb - S);
+          for (int kb = 0; ok && kb < head; ++kb) {
+            ok = wait_full(kb);
+            if (ok) mma(acc, 0, kb);
+          }
+          if (ok && head == num_kb) commit(tfull0 + 8 * acc);
+          ok = ok && wait_acc(acc ^ 1);
+          for (int kb = 0; ok && kb < head; ++kb) {
+            mma(acc ^ 1, 1, kb);
+            commit(empty0 + 8 * ((it + kb) % S));
+          }
+          for (int kb = head; ok && kb < tail; ++kb) {
+            ok = wait_full(kb);
+            if (!ok) break;
+            mma(acc, 0, kb);
+            mma(acc ^ 1, 1, kb);
+            commit(empty0 + 8 * ((it + kb) % S));
+          }
+          for (int kb = tail; ok && kb < num_kb; ++kb) {
+            ok = wait_full(kb);
+            if (ok) mma(acc, 0, kb);
+          }
+          if (ok && head < num_kb) commit(tfull0 + 8 * acc);
+          for (int kb = tail; ok && kb < num_kb; ++kb) {
+            mma(acc ^ 1, 1, kb);
+            commit(empty0 + 8 * ((it + kb) % S));
+          }
+          if (ok) commit(tfull0 + 8 * (acc ^ 1));
         }
-        if (!ok) break;
-        umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 0));
-        umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 1));
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        if (!ok) {
+          fail_code = kStatusTimeoutMma;
+          break;
+        }
+        it += num_kb;
       }
     }
   } else {
     // ---------------- epilogue (warps 2..9 of both CTAs) ----------------
     const int q = warp & 3;              // TMEM lane quarter this warp may read
-    const int half = (warp - 2) >> 2;    // which half of the tile's columns
+    const int part = (warp - 2) >> 2;    // which 128 of a half's 256 columns
     uint8_t* const stage_mem = staging + (warp - 2) * kStageWarpBytes;
     int acc = 0;
-    uint32_t acc_phase = 0;
-    for (uint32_t cnt = 0;; ++cnt) {
+    uint32_t acc_phase = 0;              // one bit per accumulator
+    bool ok = true;
+    for (uint32_t cnt = 0; ok; ++cnt) {
       const uint32_t slot = cnt % kRing;
       if (!__all_sync(0xffffffffu, mbar_wait_cluster_bounded(rfull0 + 8 * slot, (cnt / kRing) & 1u, abort_flag))) {
         fail_code = kStatusTimeoutEpilogue;
@@ -676,33 +744,38 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
       if (lane == 0) mbar_arrive_cluster(mapa_shared(rempty0 + 8 * slot, 0));
       if (e.x < 0) break;
       const OpS& op = ops[entry_op(e)];
-      const TileEpilogue tile(op.k, entry_b(e), entry_m(e) * 256 + 128 * static_cast<int>(rank) + q * 32,
-                                    entry_mirror(e), stage_mem, lane);
-      bool ready = true;
-      if (lane == 0 && e.w > 0 && tile.add_c) {
-        // C was stored by other CTAs: one lane acquires for the warp, the reads go to L2
-        ready = wait_count(done + entry_ctr(e), e.w, abort_flag);
-        if (!ready) fail_code = kStatusTimeoutPeerFlag;
+      const int halves = entry_halves<WIDE>(e);
+      for (int h = 0; h < halves; ++h) {
+        const TileEpilogue tile(op.k, entry_b(e), entry_m(e) * 256 + 128 * static_cast<int>(rank) + q * 32,
+                                entry_mirror_half(e, h), stage_mem, lane);
+        bool ready = true;
+        if (lane == 0 && e.w > 0 && tile.add_c) {
+          // C was stored by other CTAs: one lane acquires for the warp, the reads go to L2
+          ready = wait_count(done + entry_ctr(e), e.w, abort_flag);
+          if (!ready) fail_code = kStatusTimeoutPeerFlag;
+        }
+        ok = __all_sync(0xffffffffu, ready);
+        if (!ok) break;
+        const int col0 = (entry_n(e) + h) * kPairBN + part * (kPairBN / 2);
+        RawC c;
+        tile.fetch_c(c, col0);           // arrives while the product runs
+        ready = mbar_wait_bounded(tfull0 + 8 * acc, (acc_phase >> acc) & 1u, abort_flag);
+        if (!ready) fail_code = kStatusTimeoutEpilogue;
+        ok = __all_sync(0xffffffffu, ready);
+        if (!ok) break;
+        tc_fence_after_sync();
+        tile.run(tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
+                     static_cast<uint32_t>(acc * kPairBN + part * (kPairBN / 2)),
+                 col0, kPairBN / 2, c);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive_cluster(mapa_shared(tempty0 + 8 * acc, 0));   // the leader's barrier
+          red_add_release_gpu(done + entry_ctr(e), 1);              // covers the stores of the whole warp
+        }
+        acc_phase ^= 1u << acc;
+        acc ^= 1;
       }
-      if (!__all_sync(0xffffffffu, ready)) break;
-      const int col0 = entry_n(e) * kPairBN + half * (kPairBN / 2);
-      RawC c;
-      tile.fetch_c(c, col0);             // arrives while the product runs
-      if (!__all_sync(0xffffffffu, mbar_wait_bounded(tfull0 + 8 * acc, acc_phase, abort_flag))) {
-        fail_code = kStatusTimeoutEpilogue;
-        break;
-      }
-      tc_fence_after_sync();
-      tile.run(tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                   static_cast<uint32_t>(acc * kPairBN + half * (kPairBN / 2)),
-               col0, kPairBN / 2, c);
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty0 + 8 * acc, 0));   // the leader's barrier
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1u;
-      __syncwarp();
-      if (lane == 0) red_add_release_gpu(done + entry_ctr(e), 1);
     }
   }
 
@@ -711,6 +784,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
   __syncthreads();
   if (*abort_flag) {
     if (fail_code != 0 && p.status != nullptr) atomicCAS(p.status, 0, fail_code);
+    // bulk copies that may still be in flight land before the shared memory is handed on
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
     __syncthreads();
   }
@@ -743,9 +817,10 @@ ChainParams make_params(const DmuonChainArgs& a) {
   return p;
 }
 
+template <bool WIDE>
 int launch_chain_pair(const DmuonChainArgs& a, cudaStream_t stream, int sms) {
-  cudaError_t err = cudaFuncSetAttribute(chain_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         pair_smem_bytes(DMUON_CHAIN_MAX_OPS));
+  cudaError_t err = cudaFuncSetAttribute(chain_pair_kernel<WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         pair_smem_bytes<WIDE>(DMUON_CHAIN_MAX_OPS));
   if (err != cudaSuccess) return static_cast<int>(err);
   int pairs = (a.max_ctas > 0 && a.max_ctas < sms ? a.max_ctas : sms) / 2;
   if (a.total < pairs) pairs = a.total;
@@ -753,7 +828,7 @@ int launch_chain_pair(const DmuonChainArgs& a, cudaStream_t stream, int sms) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(kChainThreads, 1, 1);
-  cfg.dynamicSmemBytes = pair_smem_bytes(a.n_ops);
+  cfg.dynamicSmemBytes = pair_smem_bytes<WIDE>(a.n_ops);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -762,7 +837,7 @@ int launch_chain_pair(const DmuonChainArgs& a, cudaStream_t stream, int sms) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  err = cudaLaunchKernelEx(&cfg, chain_pair_kernel, make_params(a));
+  err = cudaLaunchKernelEx(&cfg, chain_pair_kernel<WIDE>, make_params(a));
   count_launch();
   return static_cast<int>(err != cudaSuccess ? err : cudaGetLastError());
 }
@@ -815,6 +890,6 @@ extern "C" int dmuon_chain_launch(const DmuonChainArgs* args, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   if (a.bn == 64) return launch_chain<64>(a, stream, sms);
   if (a.bn == 128) return launch_chain<128>(a, stream, sms);
-  if (a.bn == 256) return launch_chain_pair(a, stream, sms);
+  if (a.bn == 256) return a.wide ? launch_chain_pair<true>(a, stream, sms) : launch_chain_pair<false>(a, stream, sms);
   return -1;
 }

@@ -52,7 +52,9 @@ struct DmuonChainArgs {
   const int* tab;              // device: total entries of four ints, see chain_sm100.cu
   int* counters;               // device, zero between launches: ticket, exits, one per matrix
   int* status;
-  int n_ops, n_maps, total, n_counters, n_final, bn, max_ctas, pad_;
+  int n_ops, n_maps, total, n_counters, n_final, max_ctas;
+  int bn;                      // 64 or 128: 128 x bn tiles; 256: CTA pairs on 256 x 256 tiles
+  int wide;                    // CTA pairs: entries may be two tiles side by side
   struct DmuonChainFinal fin[DMUON_CHAIN_MAX_GROUPS];
 };
 

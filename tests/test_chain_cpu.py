@@ -65,9 +65,13 @@ def _interpret(specs, bn, inputs):
         rows = s.m if pr.symmetric else s.m0
         cols = s.m if pr.symmetric else s.n0
         tn, tm = CH._SUM_COLS if is_sum else bn, CH.tile_rows(bn)
-        r0, r1, c0, c1 = mt * tm, min(rows, mt * tm + tm), nt * tn, min(cols, nt * tn + tn)
-        tile(s, d, pr, ns, per, is_sum, b, split, mirror, rows, cols, r0, r1, c0, c1)
-        done[ctr] += CH.WARPS_PER_TILE * (2 if bn == CH.PAIR else 1)
+        halves = [(nt, mirror)]
+        if bn == CH.PAIR and (x >> 9) & 1:
+            halves.append((nt + 1, (x >> 10) & 1))
+        for nt, mirror in halves:
+            r0, r1, c0, c1 = mt * tm, min(rows, mt * tm + tm), nt * tn, min(cols, nt * tn + tn)
+            tile(s, d, pr, ns, per, is_sum, b, split, mirror, rows, cols, r0, r1, c0, c1)
+            done[ctr] += CH.WARPS_PER_TILE * (2 if bn == CH.PAIR else 1)
         finished_by_op[ctr][op] = done[ctr]
     # a count in the list stands for whole products: w equals the count after `after` finished
     ends = {}
@@ -80,13 +84,15 @@ def _interpret(specs, bn, inputs):
     return [d["final"] for d in buf]
 
 
+@pytest.mark.parametrize("wide", [False, True])
 @pytest.mark.parametrize("bn", [64, 128, 256])
 @pytest.mark.parametrize("shapes,formulation", [
     ([(1, 64, 96)], "gram"), ([(2, 128, 128)], "gram"), ([(1, 136, 1040)], "gram"), ([(1, 2056, 72)], "gram"),
     ([(3, 264, 200)], "direct"), ([(1, 72, 1544)], "direct"),
     ([(2, 256, 128), (1, 128, 328), (2, 72, 64)], "gram"), ([(2, 1096, 600)], "gram"), ([(30, 264, 64)], "gram"),
 ])
-def test_tile_list_computes_the_iteration(shapes, formulation, bn):
+def test_tile_list_computes_the_iteration(shapes, formulation, bn, wide, monkeypatch):
+    monkeypatch.setattr(CH, "choose_wide", lambda specs, bn: wide and bn == CH.PAIR)
     rng = np.random.default_rng(0)
     specs = [_spec(L, m0, n0, formulation) for L, m0, n0 in shapes]
     xs = []

@@ -25,6 +25,8 @@ def _rel(a, b):
     (1, 520, 520, torch.float32),         # full-width and half-width remainders of the mirror
     (5, 256, 256, torch.bfloat16),        # batch, several tickets per CTA
     (12, 1032, 1160, torch.bfloat16),     # CTA pairs, remainders in every dimension
+    (450, 136, 520, torch.bfloat16),      # two tiles an entry in the last product, K of three and nine k-blocks
+    (48, 1288, 1160, torch.float32),      # two tiles an entry, tall, K of 19 k-blocks: skewed head, middle and tail
     (75, 264, 128, torch.float32),        # CTA pairs, MN-major operands, K below one trip of the stage ring
 ])
 def test_chain_matches_64_bit_iteration(L, m0, n0, dt, formulation, monkeypatch):
@@ -48,7 +50,7 @@ def test_chain_matches_64_bit_iteration(L, m0, n0, dt, formulation, monkeypatch)
     alone = ns_sm100.newton_schulz_batched(X, coefs, restarts, 1e-7, formulation)
     torch.cuda.synchronize()
     G.check_status(_dev())
-    for i in range(L):
+    for i in sorted({0, 1, L // 2, L - 1} & set(range(L))):
         exact = NS.direct_newton_schulz(X[i].double(), coefficients=coefs, compute_dtype=torch.float64)
         limit = 1.25 * _rel(alone[i], exact) + (2e-3 if formulation == "gram" else 8e-3)
         assert _rel(out[i], exact) < limit
