@@ -142,3 +142,26 @@ def test_llama_fused_ops_match_plain_formulation():
     assert abs(res[True][0] - res[False][0]) < 2e-2
     for n, g in res[False][1].items():
         _close(res[True][1][n], g, 5e-2)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 2e-2), (torch.float16, 1e-2), (torch.float32, 1e-4)])
+@pytest.mark.parametrize("rows,chunk", [(1, 128), (256, 128), (300, 0)])
+def test_linear_cross_entropy_scaled_and_walked_twice(dtype, tol, rows, chunk):
+    """Both scale factors, and walks of a kept graph: the same gradients on every one, the
+    last walk may reuse the buffers."""
+    from dmuon_b200.ops import model_ops
+
+    torch.manual_seed(7)
+    h = torch.randn(rows, 64, device=_dev()).to(dtype).requires_grad_()
+    w = torch.randn(1001, 64, device=_dev()).mul_(0.2).to(dtype).requires_grad_()
+    y = torch.randint(0, 1001, (rows,), device=_dev())
+    if rows > 2:
+        y[::5] = -100
+    hf, wf = h.detach().float().requires_grad_(), w.detach().float().requires_grad_()
+    want = torch.autograd.grad(F.cross_entropy(F.linear(hf, wf), y, ignore_index=-100) * 3.0, (hf, wf))
+    loss = model_ops.linear_cross_entropy(h, w, y, chunk=chunk)
+    for keep in (True, True, False):
+        got = torch.autograd.grad(loss * 3.0, (h, w), retain_graph=keep)
+        for a, r in zip(got, want):
+            # 2-norm error of products and results of this type, sums in 32 bits
+            _close(a, r, tol)
