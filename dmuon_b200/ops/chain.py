@@ -230,7 +230,7 @@ def fits(specs: Sequence[GroupSpec]) -> bool:
     """Within what a plan's tables can express, matrices the kernels take."""
     if len(specs) > MAX_GROUPS or sum(s.L for s in specs) > 4096:
         return False
-    if any(s.m0 % 8 or s.n0 % 8 or s.m < 8 or not s.coefs for s in specs):
+    if any(s.L < 1 or s.m0 % 8 or s.n0 % 8 or s.m < 8 or not s.coefs for s in specs):
         return False
     # a Gram product that is split over K counts twice
     split = choose_bn(specs) != PAIR

@@ -122,6 +122,7 @@ def test_restart_variants_and_scale_factors():
 def test_limits_of_a_plan():
     assert CH.fits([_spec(1, 128, 128)])
     assert not CH.fits([_spec(1, 128, 100)])                       # pitches are multiples of eight
+    assert not CH.fits([_spec(0, 128, 128)])
     assert not CH.fits([_spec(1, 128, 128, coefs=COEFS * 20)])     # too many products
     assert not CH.fits([_spec(1, 128, 128)] * 17)
     for L, m, n in ((1, 128, 14336), (1, 1152, 4304), (8, 256, 256), (1, 128, 128)):
