@@ -92,10 +92,10 @@ def local_pow_sum(grads: list[torch.Tensor], norm_type: float, device: torch.dev
     if norm_type == 2.0 and _use_kernels(grads[0]):
         from .ops import multi_tensor as MT
 
-        acc = torch.zeros(1, dtype=torch.float32, device=device)
+        acc = torch.zeros(1, dtype=torch.float64, device=device)
         flat = [g if g.is_contiguous() else g.contiguous() for g in grads]
         MT.clip_sumsq(flat, [0] * len(flat), acc)
-        return acc[0]
+        return acc[0].float()
     norms = torch._foreach_norm([g.detach().float() for g in grads], norm_type)
     return torch.stack(norms).pow(norm_type).sum()
 

@@ -182,7 +182,12 @@ __global__ void __launch_bounds__(kBlock) clip_sumsq_kernel(const DmuonClipArgs 
   DMUON_DISPATCH(a.dtype[t], T, acc = sumsq_tensor<T>(reinterpret_cast<const T*>(a.tensor[t]), a.numel[t]));
   const float total = block_sum(acc);
   // a NaN/Inf partial sum must reach the segment total, so no "!= 0" shortcut on it
-  if (threadIdx.x == 0 && !(total == 0.f)) atomicAdd(a.seg_sumsq + a.segment[t], total);
+  // Thousands of block totals reach one word in any order: in fp32 the sum of 35 M squares came out up to
+  // 1e-6 off, by chance, in fp64 the order does not show.
+  if (threadIdx.x == 0 && !(total == 0.f)) {
+    if (a.seg_double) atomicAdd(reinterpret_cast<double*>(a.seg_sumsq) + a.segment[t], static_cast<double>(total));
+    else atomicAdd(a.seg_sumsq + a.segment[t], total);
+  }
 }
 
 template <typename T>

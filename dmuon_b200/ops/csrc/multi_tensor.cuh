@@ -83,6 +83,7 @@ struct DmuonClipArgs {
   int n;
   float* seg_sumsq;                   // [num_segments], accumulated with atomics
   const float* seg_coef;              // [num_segments], used by the scale kernel
+  int seg_double;                     // seg_sumsq holds doubles
 };
 
 // dst = cast(src * scale[slot]) ; generic multi-tensor cast/copy.

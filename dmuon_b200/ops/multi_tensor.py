@@ -50,7 +50,7 @@ class _AdamWArgs(ctypes.Structure):
 class _ClipArgs(ctypes.Structure):
     _fields_ = [
         ("tensor", _VP), ("numel", _LL), ("segment", _IA), ("dtype", _IA), ("n", ctypes.c_int),
-        ("seg_sumsq", ctypes.c_void_p), ("seg_coef", ctypes.c_void_p),
+        ("seg_sumsq", ctypes.c_void_p), ("seg_coef", ctypes.c_void_p), ("seg_double", ctypes.c_int),
     ]
 
 
@@ -230,12 +230,14 @@ def _clip_call(fn_name: str, tensors, segments, seg_sumsq, seg_coef) -> None:
             a.tensor[k], a.numel[k], a.segment[k], a.dtype[k] = t.data_ptr(), t.numel(), int(segments[i]), _DT[t.dtype]
         a.n = hi - lo
         a.seg_sumsq = seg_sumsq.data_ptr() if seg_sumsq is not None else None
+        a.seg_double = int(seg_sumsq is not None and seg_sumsq.dtype == torch.float64)
         a.seg_coef = seg_coef.data_ptr() if seg_coef is not None else None
         _check(getattr(_lib(), fn_name)(ctypes.byref(a), _stream(dev)), fn_name)
 
 
 def clip_sumsq(tensors: Sequence[torch.Tensor], segments: Sequence[int], seg_sumsq: torch.Tensor) -> None:
-    """``seg_sumsq[segments[i]] += sum(tensors[i]^2)`` in fp32."""
+    """``seg_sumsq[segments[i]] += sum(tensors[i]^2)``; totals of blocks in fp32, added
+    in the type of ``seg_sumsq`` (fp32 or fp64)."""
     _clip_call("dmuon_clip_sumsq", tensors, segments, seg_sumsq, None)
 
 
