@@ -2,9 +2,9 @@
 (``csrc/chain_sm100.cu``).
 
 A *group* is a batch of ``L`` matrices of one shape.  A *plan* covers one or more
-groups: it owns their work buffers, the encoded tensor maps, the list of products
-and the tile list, all on the device and reused by every call with the same
-shapes.  A call supplies only what changes: where the results go and the scale of
+groups: it owns their work buffers, the list of products and the tile list (on the
+device) and the encoded tensor maps (parameters of each launch), reused by every call
+with the same shapes.  A call supplies only what changes: where the results go and the scale of
 the last product (plus the operands, written into ``plan.groups[i].X`` beforehand).
 
 The tile list is ordered product by product, all groups side by side; every entry
@@ -29,6 +29,7 @@ from . import gemm as G
 
 MAX_OPS = 76
 MAX_GROUPS = 16
+MAX_MAPS = 128                # tensor maps, which travel in the kernel's parameters
 SMS = 148
 PAIRS = SMS // 2
 _KB = 64                      # inner elements per pipeline stage
@@ -226,14 +227,28 @@ def sym_tiles(specs: Sequence[GroupSpec], bn: int) -> int:
     return sum(s.L * sym_tile_count(s.m, bn) for s in specs)
 
 
+def _operands(pr: Product, bn: int) -> tuple:
+    """The tensor maps of a product's A and B: (buffer, columns and rows of the box)."""
+    return tuple((name, (64, _KB) if mn else (_KB, rows))
+                 for name, mn, rows in ((pr.A, pr.a_mn, G.BM), (pr.B, pr.b_mn, min(bn, G.BM))))
+
+
+@lru_cache(maxsize=4096)
+def _map_count(spec: GroupSpec, bn: int) -> int:
+    return len({m for pr in _products_of(spec) for m in _operands(pr, bn)})
+
+
 def fits(specs: Sequence[GroupSpec]) -> bool:
     """Within what a plan's tables can express, matrices the kernels take."""
     if len(specs) > MAX_GROUPS or sum(s.L for s in specs) > 4096:
         return False
     if any(s.L < 1 or s.m0 % 8 or s.n0 % 8 or s.m < 8 or not s.coefs for s in specs):
         return False
+    bn = choose_bn(specs)
+    if sum(_map_count(s, bn) for s in specs) > MAX_MAPS:
+        return False
     # a Gram product that is split over K counts twice
-    split = choose_bn(specs) != PAIR
+    split = bn != PAIR
     return sum(len(p) + split * sum(q.symmetric and q.A in ("X", "X2") for q in p) for p in map(_products_of, specs)) <= MAX_OPS
 
 
@@ -470,7 +485,7 @@ class Plan:
         self.tab = torch.from_numpy(entries.copy()).to(device)
         self.total = int(entries.shape[0])
         a = _Args()
-        a.ops, a.maps, a.tab = self._ops.data_ptr(), self._maps.data_ptr(), self.tab.data_ptr()
+        a.ops, a.maps, a.tab = self._ops.data_ptr(), self._maps_at, self.tab.data_ptr()
         a.counters, a.status = self.counters.data_ptr(), G.status_buffer(device).data_ptr()
         a.n_ops, a.n_maps, a.total = self.n_ops, self.n_maps, self.total
         a.n_counters, a.n_final, a.bn = self.counters.numel(), len(self.specs), self.bn
@@ -481,8 +496,7 @@ class Plan:
         maps: list[_Map] = []
         index: dict[tuple, int] = {}
 
-        def map_of(g: int, name: str, mn: bool, rows_per_tile: int) -> int:
-            box = (64, _KB) if mn else (_KB, rows_per_tile)
+        def map_of(g: int, name: str, box: tuple) -> int:
             key = (g, name, box)
             if key not in index:
                 t = self.groups[g].buffers[name]
@@ -504,8 +518,7 @@ class Plan:
             o.a_mn_major, o.b_mn_major = int(pr.a_mn), int(pr.b_mn)
             o.ab_fp16 = int(s.dtype == torch.float16)
             o.final_slot, o.splits, o.kb_per_split = -1, ns, per
-            o.map_a = -1 if is_sum else map_of(g, pr.A, pr.a_mn, G.BM)
-            o.map_b = -1 if is_sum else map_of(g, pr.B, pr.b_mn, min(self.bn, G.BM))
+            o.map_a, o.map_b = (-1, -1) if is_sum else (map_of(g, *x) for x in _operands(pr, self.bn))
             if ns > 1 and not is_sum:
                 o.alpha, o.out_kind = 1.0, 2
                 o.D, o.ldd, o.strideD = grp.partials.data_ptr(), s.m, s.m * s.m
@@ -526,13 +539,11 @@ class Plan:
                 o.D, o.ldd, o.strideD = d.data_ptr(), d.stride(1), d.stride(0)
         n = len(maps)
         marr = (_Map * n)(*maps)
-        raw = ctypes.create_string_buffer(128 * n + 64)
-        base = (ctypes.addressof(raw) + 63) & ~63
-        rc = _lib().dmuon_chain_encode_maps(marr, n, base)
+        self._maps = ctypes.create_string_buffer(128 * n + 64)
+        self._maps_at = (ctypes.addressof(self._maps) + 63) & ~63      # tensor maps are aligned to 64 bytes
+        rc = _lib().dmuon_chain_encode_maps(marr, n, self._maps_at)
         if rc != 0:
             raise RuntimeError(f"dmuon_chain_encode_maps failed with code {rc}")
-        enc = np.frombuffer(ctypes.string_at(base, 128 * n), dtype=np.uint8).copy()
-        self._maps = torch.from_numpy(enc).to(self.device)
         self._ops = torch.from_numpy(np.frombuffer(bytes(arr), dtype=np.uint8).copy()).to(self.device)
         self.n_ops, self.n_maps = len(ops), n
         self._finals = {g: pr for g, pr, *_ in ops if pr.out == "final"}

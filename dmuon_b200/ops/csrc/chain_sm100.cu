@@ -27,6 +27,7 @@
 // k-block at 64 B/clk/SM).
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <string.h>
 
 #include "chain_sm100.cuh"
 #include "gemm_epilogue.cuh"
@@ -61,16 +62,19 @@ struct OpS {
   int map_a, map_b, kb_per_split, splits;
 };
 
-// Launch parameters.
+// Launch parameters.  The tensor maps travel in them: maps in global memory that the host
+// fills by copy need a proxy fence on each map by the thread that issues the loads, in every
+// CTA, or a descriptor cached for an earlier owner of the address may be used.
 struct ChainParams {
+  CUtensorMap maps[DMUON_CHAIN_MAX_MAPS];
+  DmuonChainFinal fin[DMUON_CHAIN_MAX_GROUPS];
   const DmuonChainOp* ops;
-  const CUtensorMap* maps;
   const int4* tab;
   int* counters;
   int* status;
   int n_ops, n_maps, total, n_counters;
-  DmuonChainFinal fin[DMUON_CHAIN_MAX_GROUPS];
 };
+static_assert(sizeof(ChainParams) <= 32764, "kernel parameters are limited to 32,764 bytes");
 
 constexpr int kBarBytes = 512;
 constexpr int kStageBytesAll = kEpiWarps * kStageWarpBytes;
@@ -807,8 +811,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
 
 ChainParams make_params(const DmuonChainArgs& a) {
   ChainParams p;
+  memcpy(p.maps, a.maps, static_cast<size_t>(a.n_maps) * sizeof(CUtensorMap));
   p.ops = static_cast<const DmuonChainOp*>(a.ops);
-  p.maps = static_cast<const CUtensorMap*>(a.maps);
   p.tab = reinterpret_cast<const int4*>(a.tab);
   p.counters = a.counters;
   p.status = a.status;
@@ -877,6 +881,7 @@ extern "C" int dmuon_chain_launch(const DmuonChainArgs* args, void* stream_v) {
   const DmuonChainArgs& a = *args;
   if (a.total <= 0) return 0;
   if (a.n_ops <= 0 || a.n_ops > DMUON_CHAIN_MAX_OPS || a.n_final < 0 || a.n_final > DMUON_CHAIN_MAX_GROUPS) return -1;
+  if (a.n_maps <= 0 || a.n_maps > DMUON_CHAIN_MAX_MAPS) return -1;
   if (a.ops == nullptr || a.maps == nullptr || a.tab == nullptr || a.counters == nullptr) return -1;
   for (int i = 0; i < a.n_final; ++i) {
     const DmuonChainFinal& f = a.fin[i];

@@ -6,6 +6,7 @@ extern "C" {
 
 #define DMUON_CHAIN_MAX_OPS 76
 #define DMUON_CHAIN_MAX_GROUPS 16
+#define DMUON_CHAIN_MAX_MAPS 128
 
 // One batched product of a chain (device array; same meaning of the fields as in DmuonGemmArgs).
 struct DmuonChainOp {
@@ -48,7 +49,7 @@ struct DmuonChainMap {
 
 struct DmuonChainArgs {
   const void* ops;             // device: n_ops DmuonChainOp
-  const void* maps;            // device: n_maps encoded tensor maps (128 bytes each)
+  const void* maps;            // host: n_maps encoded tensor maps (128 bytes each), copied into the launch's parameters
   const int* tab;              // device: total entries of four ints, see chain_sm100.cu
   int* counters;               // device, zero between launches: ticket, exits, one per matrix
   int* status;

@@ -125,7 +125,21 @@ def test_limits_of_a_plan():
     assert not CH.fits([_spec(0, 128, 128)])
     assert not CH.fits([_spec(1, 128, 128, coefs=COEFS * 20)])     # too many products
     assert not CH.fits([_spec(1, 128, 128)] * 17)
+    # every tensor map is a kernel parameter: sixteen groups of the longest form that sixteen groups can have fit, more
+    # operands than MAX_MAPS do not
+    short = [_spec(1, 64 + 8 * i, 1024, coefs=COEFS[:1], restarts=()) for i in range(16)]
+    maps = [sum(CH._map_count(s, bn) for s in short) for bn in (64, 128, 256)]
+    assert CH.fits(short) and max(maps) <= CH.MAX_MAPS
     for L, m, n in ((1, 128, 14336), (1, 1152, 4304), (8, 256, 256), (1, 128, 128)):
         spl, per = CH.gram_splits(_spec(L, m, n), 128, CH.sym_tiles([_spec(L, m, n)], 128))
         kb = -(-n // 64)
         assert spl * per >= kb and (spl - 1) * per < kb and 1 <= spl <= 16
+
+
+def test_tensor_maps_are_counted(monkeypatch):
+    s = _spec(1, 128, 128)
+    ops, _ = CH.build_entries([s], CH.choose_bn([s]))
+    used = {m for _, pr, _, _, is_sum in ops if not is_sum for m in CH._operands(pr, CH.choose_bn([s]))}
+    assert len(used) == CH._map_count(s, CH.choose_bn([s]))
+    monkeypatch.setattr(CH, "MAX_MAPS", len(used) - 1)
+    assert not CH.fits([s])

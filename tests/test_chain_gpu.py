@@ -118,3 +118,24 @@ def test_chain_on_two_streams_at_once():
     for k, o in enumerate(got):
         # the norm is an atomic sum: its last bit, amplified by five fp16 steps
         assert _rel(o, want[k % 2].double()) < 2e-2
+
+
+def test_plans_that_follow_each_other_on_recycled_memory():
+    """Arenas grow, plans go and others take their addresses: every launch uses its own tensor maps."""
+    from dmuon_b200.ops import chain as CH
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+
+    coefs, dev = list(NS.DEFAULT_COEFFICIENTS), _dev()
+    torch.manual_seed(8)
+    shapes = [(64, 136), (72, 200), (256, 64), (256, 512), (512, 1032), (1032, 264), (1024, 2048), (64, 136), (256, 512)]
+    for turn in range(3):
+        for m, n in shapes:
+            x = torch.randn(1, m, n, device=dev)
+            exact = NS.direct_newton_schulz(x[0].double(), coefficients=coefs, compute_dtype=torch.float64)
+            # fp16 products of five steps on matrices that are not square (well conditioned): 0.0045 seen
+            assert _rel(ns_sm100.newton_schulz_batched(x, coefs, [2])[0], exact) < 2e-2, (turn, m, n)
+        CH.release()
+    torch.cuda.synchronize()
+    G.check_status(dev)
