@@ -1,11 +1,12 @@
 """Newton-Schulz as one launch: plans for the product-chain kernel
 (``csrc/chain_sm100.cu``).
 
-A *group* is a batch of ``L`` matrices of one shape.  A *plan* covers one or more
-groups: it owns their work buffers, the list of products and the tile list (on the
-device) and the encoded tensor maps (parameters of each launch), reused by every call
-with the same shapes.  A call supplies only what changes: where the results go and the scale of
-the last product (plus the operands, written into ``plan.groups[i].X`` beforehand).
+A *group* is a batch of ``L`` matrices of one shape.  A *program* covers one or more
+groups: the list of products and the tile list, on the device, used by every call with
+the same shapes.  A *plan* is a program with work memory: the buffers of one stream and
+the tensor maps over them (which travel as parameters of each launch).  A call supplies
+only what changes: where the results go and the scale of the last product (plus the
+operands, written into ``plan.X[i]`` beforehand).
 
 The tile list is ordered product by product, all groups side by side; every entry
 names the number of finished warps its matrix must show before the tile may start
@@ -45,7 +46,7 @@ class _Op(ctypes.Structure):
         ("map_a", _I), ("map_b", _I), ("a_mn_major", _I), ("b_mn_major", _I), ("ab_fp16", _I),
         ("M", _I), ("N", _I), ("K", _I), ("kb_per_split", _I), ("splits", _I), ("out_kind", _I), ("final_slot", _I),
         ("alpha", _F), ("beta", _F), ("diag", _F), ("pad_", _I),
-        ("alpha_vec", _VP), ("C", _VP), ("D", _VP), ("partials", _VP),
+        ("alpha_vec", _LL), ("C", _LL), ("D", _LL), ("partials", _LL),
         ("ldc", _LL), ("ldd", _LL), ("strideC", _LL), ("strideD", _LL),
     ]
 
@@ -67,7 +68,7 @@ class _Map(ctypes.Structure):
 
 class _Args(ctypes.Structure):
     _fields_ = [
-        ("ops", _VP), ("maps", _VP), ("tab", _VP), ("counters", _VP), ("status", _VP),
+        ("ops", _VP), ("maps", _VP), ("tab", _VP), ("counters", _VP), ("work", _VP), ("status", _VP),
         ("n_ops", _I), ("n_maps", _I), ("total", _I), ("n_counters", _I), ("n_final", _I),
         ("max_ctas", _I), ("bn", _I), ("wide", _I),
         ("fin", _Final * MAX_GROUPS),
@@ -240,7 +241,7 @@ def _map_count(spec: GroupSpec, bn: int) -> int:
 
 def fits(specs: Sequence[GroupSpec]) -> bool:
     """Within what a plan's tables can express, matrices the kernels take."""
-    if len(specs) > MAX_GROUPS or sum(s.L for s in specs) > 4096:
+    if len(specs) > MAX_GROUPS or sum(s.L for s in specs) > MAX_MATRICES:
         return False
     if any(s.L < 1 or s.m0 % 8 or s.n0 % 8 or s.m < 8 or not s.coefs for s in specs):
         return False
@@ -320,21 +321,33 @@ def gram_splits(spec: GroupSpec, bn: int, tiles_all: int) -> tuple[int, int]:
     return -(-num_kb // per), per
 
 
+def _up(n: int) -> int:
+    return -(-n // 1024) * 1024
+
+
+#: matrices of a plan; their counters and sums of squares stand at the head of the work memory
+MAX_MATRICES = 4096
+CONTROL_BYTES = _up(4 * (2 + 2 * MAX_MATRICES))
+
+
 class Arena:
     """Work memory of one stream.  Plans of a stream use it one after the other (the
     operands are written, the chain runs, the result leaves), so they share it; the
-    lock spans those steps on the host."""
+    lock spans those steps on the host.
+
+    At its head lie ticket, exits, one counter per matrix and the sums of squares of the
+    plan that runs: all zero between calls, the kernel clears them itself."""
 
     def __init__(self, nbytes: int, device):
         self.lock = threading.RLock()
         self.buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        self.used = 0
+        self.control = self.buf[:CONTROL_BYTES].view(torch.int32)
+        self.control.zero_()
+        self.dirty = False          # a call was abandoned half-way: the head has to be cleared
 
-    def take(self, shape, dtype) -> torch.Tensor:
+    def at(self, offset: int, shape, dtype) -> torch.Tensor:
         n = math.prod(shape) * torch.empty(0, dtype=dtype).element_size()
-        t = self.buf[self.used : self.used + n].view(dtype).view(shape)
-        self.used += -(-n // 1024) * 1024
-        return t
+        return self.buf[offset : offset + n].view(dtype).view(shape)
 
 
 def _buffer_shapes(spec: GroupSpec, splits: int) -> dict:
@@ -347,26 +360,26 @@ def _buffer_shapes(spec: GroupSpec, splits: int) -> dict:
     return out
 
 
-def plan_bytes(specs: Sequence[GroupSpec]) -> int:
-    bn = choose_bn(specs)
+def _layout(specs: Sequence[GroupSpec], bn: int) -> tuple[list[dict], int, int, int]:
+    """Where everything lies in the work memory: per group ``{buffer: (offset, shape,
+    dtype)}``, the offsets of the two vectors of factors per matrix, and the bytes in all."""
     tiles = sym_tiles(specs, bn)
-    total = 0
+    n = sum(s.L for s in specs)
+    vec = CONTROL_BYTES
+    vec2 = vec + _up(4 * n)
+    at = vec2 + _up(4 * n)
+    groups = []
     for s in specs:
-        for shape, dtype in _buffer_shapes(s, gram_splits(s, bn, tiles)[0]).values():
-            n = math.prod(shape) * (4 if dtype == torch.float32 else 2)
-            total += -(-n // 1024) * 1024
-    return total
+        group = {}
+        for name, (shape, dtype) in _buffer_shapes(s, gram_splits(s, bn, tiles)[0]).items():
+            group[name] = (at, shape, dtype)
+            at += _up(math.prod(shape) * (4 if dtype == torch.float32 else 2))
+        groups.append(group)
+    return groups, vec, vec2, at
 
 
-class Group:
-    """Work buffers of one group."""
-
-    def __init__(self, spec: GroupSpec, splits: int, arena: Arena):
-        self.spec = spec
-        arena_of = _buffer_shapes(spec, splits)
-        self.buffers = {name: arena.take(shape, dtype) for name, (shape, dtype) in arena_of.items()}
-        self.X = self.buffers["X"]
-        self.partials: Optional[torch.Tensor] = self.buffers.get("partials")
+def plan_bytes(specs: Sequence[GroupSpec]) -> int:
+    return _layout(specs, choose_bn(specs))[3]
 
 
 def _two_wide(e: np.ndarray) -> np.ndarray:
@@ -454,63 +467,52 @@ def build_entries(specs: Sequence[GroupSpec], bn: int):
     return ops, (entries & 0xFFFFFFFF).astype(np.uint32).view(np.int32)
 
 
-class Plan:
-    def __init__(self, specs: Sequence[GroupSpec], device: torch.device, arena: Arena):
+class Program:
+    """What a plan knows before it has work memory: the operations (with offsets into that
+    memory), the tile list and the operands' tensor maps.  The lists lie on the device in
+    one piece and serve every stream."""
+
+    def __init__(self, specs: Sequence[GroupSpec], device: torch.device):
         self.specs = tuple(specs)
         self.device = device
+        self.captured = False       # a CUDA graph names the lists
         self.bn = choose_bn(self.specs)
-        self.arena = arena
-        self.lock = arena.lock
         self.wide = choose_wide(self.specs, self.bn)
-        tiles = sym_tiles(self.specs, self.bn)
-        arena.used = 0
-        self.groups = [Group(s, gram_splits(s, self.bn, tiles)[0], arena) for s in self.specs]
+        self.groups, self.vec, self.vec2, self.nbytes = _layout(self.specs, self.bn)
         self.n_matrices = sum(s.L for s in self.specs)
+        assert self.n_matrices <= MAX_MATRICES
         self.first = [0]
         for s in self.specs:
             self.first.append(self.first[-1] + s.L)
-        n = self.n_matrices
-        # ticket, exits, one counter per matrix, then the sums of squares: all cleared by the kernel itself
-        self.counters = torch.zeros(2 + 2 * n, dtype=torch.int32, device=device)
-        self.sumsq = self.counters[2 + n :].view(torch.float32)
-        self.vec = torch.empty(n, dtype=torch.float32, device=device)
-        self.vec2 = torch.empty(n, dtype=torch.float32, device=device)
-        # the power of two that keeps fp16 operands clear of the subnormals, per matrix
-        self.k = torch.tensor([fp16_prescale(s.m0, s.n0) for s in self.specs for _ in range(s.L)], device=device)
-        self.dirty = False          # a call was abandoned half-way: the counters have to be cleared
-        self.pinned = False         # captured in a CUDA graph
         ops, entries = build_entries(self.specs, self.bn)
         assert len(ops) <= MAX_OPS
-        self._encode(ops)
-        self.tab = torch.from_numpy(entries.copy()).to(device)
-        self.total = int(entries.shape[0])
-        a = _Args()
-        a.ops, a.maps, a.tab = self._ops.data_ptr(), self._maps_at, self.tab.data_ptr()
-        a.counters, a.status = self.counters.data_ptr(), G.status_buffer(device).data_ptr()
-        a.n_ops, a.n_maps, a.total = self.n_ops, self.n_maps, self.total
-        a.n_counters, a.n_final, a.bn = self.counters.numel(), len(self.specs), self.bn
-        a.wide = int(self.wide)
-        self._args = a
+        self.n_ops, self.total = len(ops), int(entries.shape[0])
+        self.maps: list[tuple] = []          # (group, buffer, box)
+        self.finals = {g: pr for g, pr, *_ in ops if pr.out == "final"}
+        # the power of two that keeps fp16 operands clear of the subnormals, per matrix
+        k = np.repeat([fp16_prescale(s.m0, s.n0) for s in self.specs], [s.L for s in self.specs]).astype(np.float32)
+        parts = [np.frombuffer(bytes(self._operations(ops)), dtype=np.uint8), entries.view(np.uint8).reshape(-1),
+                 k.view(np.uint8)]
+        at = np.cumsum([0] + [_up(len(x)) for x in parts])
+        host = np.zeros(at[-1], dtype=np.uint8)
+        for lo, x in zip(at, parts):
+            host[lo : lo + len(x)] = x
+        self.lists = torch.from_numpy(host).to(device)
+        self.ops_at, self.tab_at = (self.lists.data_ptr() + int(lo) for lo in at[:2])
+        self.k = self.lists[at[2] : at[2] + len(parts[2])].view(torch.float32)
 
-    def _encode(self, ops) -> None:
-        maps: list[_Map] = []
+    def _operations(self, ops):
         index: dict[tuple, int] = {}
 
-        def map_of(g: int, name: str, box: tuple) -> int:
-            key = (g, name, box)
+        def map_of(key: tuple) -> int:
             if key not in index:
-                t = self.groups[g].buffers[name]
-                L, r, c = t.shape
-                m = _Map()
-                m.base, m.rows, m.cols, m.batch, m.ld, m.batch_stride = t.data_ptr(), r, c, L, c, r * c
-                m.fp16, m.box_cols, m.box_rows = int(t.dtype == torch.float16), box[0], box[1]
-                index[key] = len(maps)
-                maps.append(m)
+                index[key] = len(self.maps)
+                self.maps.append(key)
             return index[key]
 
         arr = (_Op * len(ops))()
         for i, (g, pr, ns, per, is_sum) in enumerate(ops):
-            s, grp = self.specs[g], self.groups[g]
+            s, bufs = self.specs[g], self.groups[g]
             o = arr[i]
             o.M = s.m if pr.symmetric else s.m0
             o.N = s.m if pr.symmetric else s.n0
@@ -518,51 +520,79 @@ class Plan:
             o.a_mn_major, o.b_mn_major = int(pr.a_mn), int(pr.b_mn)
             o.ab_fp16 = int(s.dtype == torch.float16)
             o.final_slot, o.splits, o.kb_per_split = -1, ns, per
-            o.map_a, o.map_b = (-1, -1) if is_sum else (map_of(g, *x) for x in _operands(pr, self.bn))
+            o.map_a, o.map_b = (-1, -1) if is_sum else (map_of((g, *x)) for x in _operands(pr, self.bn))
+            o.alpha_vec = o.C = o.D = o.partials = -1
             if ns > 1 and not is_sum:
                 o.alpha, o.out_kind = 1.0, 2
-                o.D, o.ldd, o.strideD = grp.partials.data_ptr(), s.m, s.m * s.m
+                o.D, o.ldd, o.strideD = bufs["partials"][0], s.m, s.m * s.m
                 continue
             o.alpha, o.beta, o.diag = pr.alpha, pr.beta, pr.diag
             o.out_kind = G._OUT_KIND[s.dtype]
             if pr.vec is not None:
-                o.alpha_vec = (self.vec if pr.vec == "vec" else self.vec2).data_ptr() + 4 * self.first[g]
+                o.alpha_vec = (self.vec if pr.vec == "vec" else self.vec2) + 4 * self.first[g]
             if is_sum:
-                o.partials = grp.partials.data_ptr()
+                o.partials = bufs["partials"][0]
             if pr.C is not None:
-                c = grp.buffers[pr.C]
-                o.C, o.ldc, o.strideC = c.data_ptr(), c.stride(1), c.stride(0)
+                o.C, (_, rows, o.ldc), _ = bufs[pr.C]
+                o.strideC = rows * o.ldc
             if pr.out == "final":
                 o.final_slot = g
             else:
-                d = grp.buffers[pr.out]
-                o.D, o.ldd, o.strideD = d.data_ptr(), d.stride(1), d.stride(0)
-        n = len(maps)
-        marr = (_Map * n)(*maps)
-        self._maps = ctypes.create_string_buffer(128 * n + 64)
-        self._maps_at = (ctypes.addressof(self._maps) + 63) & ~63      # tensor maps are aligned to 64 bytes
-        rc = _lib().dmuon_chain_encode_maps(marr, n, self._maps_at)
+                o.D, (_, rows, o.ldd), _ = bufs[pr.out]
+                o.strideD = rows * o.ldd
+        return arr
+
+    def encode(self, base: int):
+        """The tensor maps over the work memory at ``base``: (their owner, their address)."""
+        n = len(self.maps)
+        marr = (_Map * n)()
+        for m, (g, name, box) in zip(marr, self.maps):
+            offset, (L, r, c), dtype = self.groups[g][name]
+            m.base, m.rows, m.cols, m.batch, m.ld, m.batch_stride = base + offset, r, c, L, c, r * c
+            m.fp16, m.box_cols, m.box_rows = int(dtype == torch.float16), box[0], box[1]
+        raw = ctypes.create_string_buffer(128 * n + 64)
+        at = (ctypes.addressof(raw) + 63) & ~63      # tensor maps are aligned to 64 bytes
+        rc = _lib().dmuon_chain_encode_maps(marr, n, at)
         if rc != 0:
             raise RuntimeError(f"dmuon_chain_encode_maps failed with code {rc}")
-        self._ops = torch.from_numpy(np.frombuffer(bytes(arr), dtype=np.uint8).copy()).to(self.device)
-        self.n_ops, self.n_maps = len(ops), n
-        self._finals = {g: pr for g, pr, *_ in ops if pr.out == "final"}
+        return raw, at
+
+
+class Plan:
+    """A program and its work memory."""
+
+    def __init__(self, program: Program, arena: Arena):
+        self.program, self.arena, self.lock = program, arena, arena.lock
+        self.specs, self.device, self.n_matrices, self.k = program.specs, program.device, program.n_matrices, program.k
+        n = self.n_matrices
+        self.X = [arena.at(*g["X"]) for g in program.groups]
+        self.sumsq = arena.control[2 + n : 2 + 2 * n].view(torch.float32)
+        self.vec = arena.at(program.vec, (n,), torch.float32)
+        self.vec2 = arena.at(program.vec2, (n,), torch.float32)
+        base = arena.buf.data_ptr()
+        self._maps, maps_at = program.encode(base)
+        a = _Args()
+        a.ops, a.maps, a.tab = program.ops_at, maps_at, program.tab_at
+        a.counters, a.work, a.status = base, base, G.status_buffer(self.device).data_ptr()
+        a.n_ops, a.n_maps, a.total = program.n_ops, len(program.maps), program.total
+        a.n_counters, a.n_final, a.bn, a.wide = 2 + 2 * n, len(self.specs), program.bn, int(program.wide)
+        self._args = a
 
     def begin(self) -> None:
         """Call before the sums of squares are accumulated."""
-        if self.dirty:
-            self.counters.zero_()
-        self.dirty = True
+        if self.arena.dirty:
+            self.arena.control.zero_()
+        self.arena.dirty = True
 
     def run(self, finals: Sequence[dict]) -> None:
         """Launch the chain on the current stream.  ``finals[g]``: ``out`` (a
         ``[L, m0, n0]`` tensor) or ``out_tab`` / ``c_tab`` / ``out2_tab`` (device tables
         of addresses, multiples of 16 bytes) with ``out_dtype``; ``alpha`` multiplies the plan's own factor."""
-        a = self._args
+        a, program = self._args, self.program
         for g, f in enumerate(finals):
-            s, pr, fin = self.specs[g], self._finals[g], a.fin[g]
+            s, pr, fin = self.specs[g], program.finals[g], a.fin[g]
             fin.alpha = float(f.get("alpha", 1.0)) * pr.alpha
-            fin.alpha_vec = self.vec.data_ptr() + 4 * self.first[g] if pr.vec is not None else None
+            fin.alpha_vec = self.vec.data_ptr() + 4 * program.first[g] if pr.vec is not None else None
             fin.C = fin.C_tab = fin.D = fin.D_tab = fin.D2_tab = None
             fin.ldc = fin.ldd = fin.ldd2 = s.n0
             fin.strideC = fin.strideD = s.m0 * s.n0
@@ -572,7 +602,7 @@ class Plan:
                 fin.D, fin.out_kind = out.data_ptr(), G._OUT_KIND[out.dtype]
                 if pr.C is not None:
                     assert out.dtype == s.dtype
-                    fin.C, fin.beta = self.groups[g].buffers[pr.C].data_ptr(), pr.beta
+                    fin.C, fin.beta = self.arena.buf.data_ptr() + program.groups[g][pr.C][0], pr.beta
                 continue
             assert pr.C is None
             fin.D_tab, fin.out_kind = f["out_tab"].data_ptr(), G._OUT_KIND[f["out_dtype"]]
@@ -584,7 +614,7 @@ class Plan:
         rc = _lib().dmuon_chain_launch(ctypes.byref(a), stream)
         if rc != 0:
             raise RuntimeError(f"dmuon_chain_launch failed with code {rc}")
-        self.dirty = False
+        self.arena.dirty = False
 
 
 # ---------------------------------------------------------------------------- plans that are kept
@@ -592,6 +622,7 @@ class Plan:
 MAX_PLAN_BYTES = 6 << 30
 MAX_PLANS = 256
 MAX_ARENAS = 8
+_programs: "OrderedDict[tuple, Program]" = OrderedDict()
 _plans: "OrderedDict[tuple, Plan]" = OrderedDict()
 _arenas: "OrderedDict[tuple, Arena]" = OrderedDict()
 _lock = threading.RLock()
@@ -603,51 +634,74 @@ def possible(specs: tuple[GroupSpec, ...]) -> bool:
     return fits(specs) and plan_bytes(specs) <= MAX_PLAN_BYTES
 
 
+def _program_for(sig: tuple) -> Program:
+    p = _programs.get(sig)
+    if p is None:
+        if len(_programs) >= MAX_PLANS:
+            _programs.pop(next((k for k, q in _programs.items() if not q.captured), None), None)
+        p = _programs[sig] = Program(*sig)
+    _programs.move_to_end(sig)
+    return p
+
+
+def _arena_for(where: tuple, nbytes: int, device: torch.device) -> Arena:
+    arena = _arenas.get(where)
+    if arena is None or arena.buf.numel() < nbytes:
+        # plans on the smaller memory go: only their work memory's addresses are lost, the programs stay
+        _drop(lambda k: k[1] == where)
+        _arenas.pop(where, None)
+        arena = None
+        arena = _arenas[where] = Arena(nbytes, device)
+    _arenas.move_to_end(where)
+    while len(_arenas) > MAX_ARENAS:
+        old, _ = _arenas.popitem(last=False)
+        _drop(lambda k: k[1] == old)
+    return arena
+
+
 def plan_for(specs: Sequence[GroupSpec], device: torch.device) -> Optional[Plan]:
-    """The plan of these groups for the current stream (work memory is never shared
-    between streams).  While a CUDA graph is captured nothing can be uploaded:
-    then a plan that an earlier call made on another stream is taken and kept for
-    good, and ``None`` is returned if there is none."""
-    sig = (tuple(specs), device.index)
+    """The plan of these groups for the current stream: work memory is never shared
+    between streams, nor between a captured call and any other.
+
+    While a CUDA graph is captured, the work memory is allocated like every other
+    temporary of the captured call: it belongs to the graph, whatever stream replays it,
+    and the head is cleared by the graph itself.  The program is one that an earlier call
+    made (nothing can be uploaded now) and is kept for good, because the graph names its
+    lists; ``None`` if there is none, or too many are kept already."""
+    sig = (tuple(specs), device)
     if torch.cuda.is_current_stream_capturing():
         with _lock:
-            for k, p in _plans.items():
-                if k[0] == sig:
-                    p.pinned = True
-                    return p
-        return None
+            program = _programs.get(sig)
+            if program is None:
+                return None
+            if not program.captured and sum(p.captured for p in _programs.values()) >= MAX_PLANS // 2:
+                return None
+            program.captured = True
+        return Plan(program, Arena(program.nbytes, device))
     where = (device.index, torch._C._cuda_getCurrentRawStream(device.index))
     key = (sig, where)
     with _lock:
         p = _plans.get(key)
-        if p is not None:
-            _plans.move_to_end(key)
-            return p
-        need = plan_bytes(specs)
-        arena = _arenas.get(where)
-        if arena is None or arena.buf.numel() < need:
-            # plans made on the smaller memory go (a captured one keeps its own alive)
-            _drop(lambda k, q: k[1] == where and not q.pinned)
-            _arenas.pop(where, None)
-            arena = None
-            arena = _arenas[where] = Arena(need, device)
-        _arenas.move_to_end(where)
-        while len(_arenas) > MAX_ARENAS:
-            old, _ = _arenas.popitem(last=False)
-            _drop(lambda k, q: k[1] == old and not q.pinned)
-        if len(_plans) >= MAX_PLANS:
-            oldest = next((k for k, q in _plans.items() if not q.pinned), None)
-            _plans.pop(oldest, None)
-        p = _plans[key] = Plan(specs, device, arena)
+        if p is None:
+            program = _program_for(sig)
+            # freed only when this stream has finished with them
+            program.lists.record_stream(torch.cuda.current_stream(device))
+            p = Plan(program, _arena_for(where, program.nbytes, device))
+            if len(_plans) >= MAX_PLANS:
+                _plans.popitem(last=False)
+            _plans[key] = p
+        _plans.move_to_end(key)
         return p
 
 
 def _drop(which) -> None:
-    for k in [k for k, q in _plans.items() if which(k, q)]:
+    for k in [k for k in _plans if which(k)]:
         del _plans[k]
 
 
 def release() -> None:
     with _lock:
+        for k in [k for k, p in _programs.items() if not p.captured]:
+            del _programs[k]
         _plans.clear()
         _arenas.clear()

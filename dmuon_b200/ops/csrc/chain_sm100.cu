@@ -71,6 +71,7 @@ struct ChainParams {
   const DmuonChainOp* ops;
   const int4* tab;
   int* counters;
+  char* work;
   int* status;
   int n_ops, n_maps, total, n_counters;
 };
@@ -103,13 +104,18 @@ __device__ __forceinline__ void entry_k_range(const OpS& op, const int4& e, int&
   }
 }
 
+template <typename T>
+__device__ __forceinline__ T* work_at(const ChainParams& p, long long offset) {
+  return offset < 0 ? nullptr : reinterpret_cast<T*>(p.work + offset);
+}
+
 __device__ __forceinline__ void build_op(OpS& s, const DmuonChainOp& o, const ChainParams& p) {
   KParams k = {};
   k.M = o.M; k.N = o.N; k.K = o.K;
   k.a_mn_major = o.a_mn_major; k.b_mn_major = o.b_mn_major; k.ab_fp16 = o.ab_fp16;
   k.alpha = o.alpha; k.beta = o.beta; k.diag = o.diag;
-  k.alpha_vec = o.alpha_vec;
-  k.C = o.C; k.D = o.D;
+  k.alpha_vec = work_at<const float>(p, o.alpha_vec);
+  k.C = work_at<const void>(p, o.C); k.D = work_at<void>(p, o.D);
   k.ldc = o.ldc; k.ldd = o.ldd;
   k.strideC = o.strideC; k.strideD = o.strideD;
   k.out_kind = o.out_kind;
@@ -125,7 +131,7 @@ __device__ __forceinline__ void build_op(OpS& s, const DmuonChainOp& o, const Ch
   }
   if (k.C == nullptr && k.C_tab == nullptr) k.beta = 0.f;
   s.k = k;
-  s.partials = o.partials;
+  s.partials = work_at<const float>(p, o.partials);
   s.map_a = o.map_a; s.map_b = o.map_b;
   s.kb_per_split = o.kb_per_split; s.splits = o.splits;
 }
@@ -815,6 +821,7 @@ ChainParams make_params(const DmuonChainArgs& a) {
   p.ops = static_cast<const DmuonChainOp*>(a.ops);
   p.tab = reinterpret_cast<const int4*>(a.tab);
   p.counters = a.counters;
+  p.work = static_cast<char*>(a.work);
   p.status = a.status;
   p.n_ops = a.n_ops; p.n_maps = a.n_maps; p.total = a.total; p.n_counters = a.n_counters;
   for (int i = 0; i < DMUON_CHAIN_MAX_GROUPS; ++i) p.fin[i] = a.fin[i];
@@ -882,7 +889,7 @@ extern "C" int dmuon_chain_launch(const DmuonChainArgs* args, void* stream_v) {
   if (a.total <= 0) return 0;
   if (a.n_ops <= 0 || a.n_ops > DMUON_CHAIN_MAX_OPS || a.n_final < 0 || a.n_final > DMUON_CHAIN_MAX_GROUPS) return -1;
   if (a.n_maps <= 0 || a.n_maps > DMUON_CHAIN_MAX_MAPS) return -1;
-  if (a.ops == nullptr || a.maps == nullptr || a.tab == nullptr || a.counters == nullptr) return -1;
+  if (a.ops == nullptr || a.maps == nullptr || a.tab == nullptr || a.counters == nullptr || a.work == nullptr) return -1;
   for (int i = 0; i < a.n_final; ++i) {
     const DmuonChainFinal& f = a.fin[i];
     if ((reinterpret_cast<uintptr_t>(f.D) & 15) || (reinterpret_cast<uintptr_t>(f.C) & 15)) return -1;

@@ -9,6 +9,8 @@ extern "C" {
 #define DMUON_CHAIN_MAX_MAPS 128
 
 // One batched product of a chain (device array; same meaning of the fields as in DmuonGemmArgs).
+// What it reads and writes lies in the work memory that a launch names, so one list serves every
+// stream: alpha_vec, C, D and partials are byte offsets into it, -1 where there is none.
 struct DmuonChainOp {
   int map_a, map_b;            // indices into the chain's tensor maps; map_a < 0: sum of partial products
   int a_mn_major, b_mn_major, ab_fp16;
@@ -19,10 +21,8 @@ struct DmuonChainOp {
   int final_slot;              // >= 0: output, scale and pointer tables come from the launch (DmuonChainFinal)
   float alpha, beta, diag;
   int pad_;
-  const float* alpha_vec;
-  const void* C;
-  void* D;
-  const float* partials;       // input of a sum
+  long long alpha_vec, C, D;
+  long long partials;          // input of a sum
   long long ldc, ldd, strideC, strideD;
 };
 
@@ -52,6 +52,7 @@ struct DmuonChainArgs {
   const void* maps;            // host: n_maps encoded tensor maps (128 bytes each), copied into the launch's parameters
   const int* tab;              // device: total entries of four ints, see chain_sm100.cu
   int* counters;               // device, zero between launches: ticket, exits, one per matrix
+  void* work;                  // device: what the operations' offsets count from
   int* status;
   int n_ops, n_maps, total, n_counters, n_final, max_ctas;
   int bn;                      // 64 or 128: 128 x bn tiles; 256: CTA pairs on 256 x 256 tiles

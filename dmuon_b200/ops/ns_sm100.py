@@ -298,7 +298,7 @@ def newton_schulz_batched(
         spec = _spec_of(L, m0, n0, cd, formulation, tuple(map(tuple, coefs)), tuple(restarts), 1.0 / K, False)
         plan = CH.plan_for((spec,), X_in.device) if _chain_pays((spec,)) else None
         if plan is not None:
-            mats, X = [X_in[i] for i in range(L)], plan.groups[0].X
+            mats, X = [X_in[i] for i in range(L)], plan.X[0]
             res = out if formulation == "gram" or out.dtype == cd else torch.empty_like(out, dtype=cd)
             with plan.lock:
                 plan.begin()
@@ -482,7 +482,7 @@ def _muon_update_chain(plan: "CH.Plan", jobs: Sequence[UpdateJob]) -> None:
         if len(_prescales) > 4096:
             _prescales.clear()
         pre = torch.empty_like(plan.vec)
-    operands = [grp.X[i] for grp in plan.groups for i in range(grp.spec.L)]
+    operands = [x for X in plan.X for x in X]
     stage = [torch.empty(x.shape, dtype=torch.float32, device=x.device) for x in operands] if fresh else operands
     slots = range(plan.n_matrices)
     plan.begin()

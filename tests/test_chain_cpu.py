@@ -143,3 +143,67 @@ def test_tensor_maps_are_counted(monkeypatch):
     assert len(used) == CH._map_count(s, CH.choose_bn([s]))
     monkeypatch.setattr(CH, "MAX_MAPS", len(used) - 1)
     assert not CH.fits([s])
+
+
+class _Memory:
+    """Stands for an arena or a program: only who holds which."""
+
+    def __init__(self, *args):
+        self.args, self.captured, self.lists = args, False, self
+        self.specs = args[0] if isinstance(args[0], tuple) else ()
+        self.nbytes = CH.plan_bytes(self.specs) if self.specs else args[0]
+        self.buf = self
+
+    def numel(self):
+        return self.nbytes
+
+    def record_stream(self, stream):
+        pass
+
+
+@pytest.fixture
+def streams(monkeypatch):
+    """``plan_for`` without a device: the current stream and whether it captures are set by the test."""
+    now = {"stream": 1, "capturing": False}
+    monkeypatch.setattr(CH, "Program", _Memory)
+    monkeypatch.setattr(CH, "Arena", _Memory)
+    monkeypatch.setattr(CH, "Plan", lambda program, arena: type("P", (), dict(program=program, arena=arena)))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: now["capturing"])
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: now["stream"])
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: now["stream"], raising=False)
+    for pool in ("_programs", "_plans", "_arenas"):
+        monkeypatch.setattr(CH, pool, type(getattr(CH, pool))())
+    return now
+
+
+def test_captured_calls_have_work_memory_of_their_own(streams):
+    dev = torch.device("cuda", 0)
+    small, large = [_spec(1, 64, 128)], [_spec(1, 256, 512)]
+    eager = CH.plan_for(small, dev)
+    assert CH.plan_for(small, dev) is eager
+    CH.plan_for(large, dev)                       # the arena grows: the smaller shape's plan goes with it
+    streams.update(stream=7, capturing=True)
+    first, second = CH.plan_for(small, dev), CH.plan_for(small, dev)
+    streams["capturing"] = False
+    plans = [first, second]
+    for s in (1, 7):
+        streams["stream"] = s
+        plans += [CH.plan_for(large, dev), CH.plan_for(small, dev)]
+    assert first.program is second.program is eager.program is plans[3].program is plans[5].program
+    # two plans of one stream share its arena; nothing else shares anything
+    assert plans[2].arena is plans[3].arena and plans[4].arena is plans[5].arena
+    assert len({id(p.arena) for p in plans}) == 4
+    assert not {id(p.arena) for p in (first, second)} & {id(a) for a in CH._arenas.values()}
+    # the lists a graph names stay, whatever is given back or replaced
+    CH.release()
+    assert list(CH._programs.values()) == [first.program] and not CH._plans and not CH._arenas
+    for i in range(CH.MAX_PLANS + 8):
+        CH.plan_for([_spec(1, 64, 8 * (i + 20))], dev)
+    assert len(CH._programs) <= CH.MAX_PLANS and first.program in CH._programs.values()
+    assert len(CH._plans) <= CH.MAX_PLANS
+
+
+def test_capture_without_an_earlier_call_has_no_plan(streams):
+    streams["capturing"] = True
+    assert CH.plan_for([_spec(1, 64, 128)], torch.device("cuda", 0)) is None
+    assert not CH._programs

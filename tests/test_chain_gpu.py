@@ -139,3 +139,78 @@ def test_plans_that_follow_each_other_on_recycled_memory():
         CH.release()
     torch.cuda.synchronize()
     G.check_status(dev)
+
+
+def _graph_of(fn, x):
+    static_in = x.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        static_out = fn(static_in)
+    return graph, static_in, static_out
+
+
+def test_shapes_called_in_ascending_order_can_be_captured():
+    """Work memory that grew for a larger shape does not take a smaller one's plan from a later capture."""
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+    from dmuon_b200.optim import ns_graph
+
+    coefs, dev = list(NS.DEFAULT_COEFFICIENTS), _dev()
+    torch.manual_seed(9)
+
+    def fn(x):
+        return ns_sm100.newton_schulz_batched(x, coefs, [2])
+
+    # sizes of no other test: the separate launches have no tile lists of them either.  bf16: the norm's last bit,
+    # which is an atomic sum, does not show
+    xs = [torch.randn(1, m, n, device=dev).bfloat16() for m, n in ((264, 1096), (968, 2120), (1416, 2664))]
+    want = [fn(x) for x in xs]
+    graphs = [_graph_of(fn, x) for x in xs]
+    cache = ns_graph.NSGraphCache()
+    for turn in range(3):
+        for x, w, (graph, static_in, static_out) in zip(xs, want, graphs):
+            static_in.copy_(x)
+            graph.replay()
+            assert _rel(static_out, w.double()) < 1e-2
+            assert _rel(cache.run(tuple(x.shape), fn, x), w.double()) < 1e-2
+    torch.cuda.synchronize()
+    G.check_status(dev)
+    assert cache.stats() == dict(keys=3, captures=3, replays=6, failed=0)
+
+
+def test_replays_beside_eager_calls_on_other_streams():
+    """A graph's work memory and counters are its own: two graphs of one shape and eager calls of this and
+    another shape run at once on four streams."""
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+
+    coefs, dev = list(NS.DEFAULT_COEFFICIENTS), _dev()
+    torch.manual_seed(10)
+
+    def fn(x):
+        return ns_sm100.newton_schulz_batched(x, coefs, [2])
+
+    a = [torch.randn(1, 520, 1160, device=dev).bfloat16() for _ in range(3)]
+    b = torch.randn(1, 776, 1288, device=dev).bfloat16()
+    want, want_b = [fn(x) for x in a], fn(b)
+    graphs = [_graph_of(fn, x) for x in a[:2]]
+    streams = [torch.cuda.Stream(dev) for _ in range(3)]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(10):
+        for k, (graph, _, static_out) in enumerate(graphs):
+            with torch.cuda.stream(streams[k]):
+                graph.replay()
+                got.append((static_out.clone(), want[k]))
+        with torch.cuda.stream(streams[2]):
+            got.append((fn(b), want_b))
+            got.append((fn(a[2]), want[2]))
+        got.append((fn(b), want_b))
+        got.append((fn(a[2]), want[2]))
+    torch.cuda.synchronize()
+    G.check_status(dev)
+    for out, w in got:
+        assert _rel(out, w.double()) < 1e-2
