@@ -666,15 +666,14 @@ def plan_for(specs: Sequence[GroupSpec], device: torch.device) -> Optional[Plan]
     While a CUDA graph is captured, the work memory is allocated like every other
     temporary of the captured call: it belongs to the graph, whatever stream replays it,
     and the head is cleared by the graph itself.  The program is one that an earlier call
-    made (nothing can be uploaded now) and is kept for good, because the graph names its
-    lists; ``None`` if there is none, or too many are kept already."""
+    made (nothing can be uploaded now; ``None`` if there is none) and is kept for good,
+    because the graph names its lists: 16 bytes a tile, far less than the work memory that
+    the graph itself holds."""
     sig = (tuple(specs), device)
     if torch.cuda.is_current_stream_capturing():
         with _lock:
             program = _programs.get(sig)
             if program is None:
-                return None
-            if not program.captured and sum(p.captured for p in _programs.values()) >= MAX_PLANS // 2:
                 return None
             program.captured = True
         return Plan(program, Arena(program.nbytes, device))
