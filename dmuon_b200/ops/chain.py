@@ -360,14 +360,15 @@ def _buffer_shapes(spec: GroupSpec, splits: int) -> dict:
     return out
 
 
-def _layout(specs: Sequence[GroupSpec], bn: int) -> tuple[list[dict], int, int, int]:
+def _layout(specs: Sequence[GroupSpec], bn: int) -> tuple[list[dict], tuple, int]:
     """Where everything lies in the work memory: per group ``{buffer: (offset, shape,
-    dtype)}``, the offsets of the two vectors of factors per matrix, and the bytes in all."""
+    dtype)}``, the offsets of three words per matrix (two factors, a flag), and the bytes in all."""
     tiles = sym_tiles(specs, bn)
     n = sum(s.L for s in specs)
     vec = CONTROL_BYTES
     vec2 = vec + _up(4 * n)
-    at = vec2 + _up(4 * n)
+    again = vec2 + _up(4 * n)
+    at = again + _up(4 * n)
     groups = []
     for s in specs:
         group = {}
@@ -375,11 +376,11 @@ def _layout(specs: Sequence[GroupSpec], bn: int) -> tuple[list[dict], int, int, 
             group[name] = (at, shape, dtype)
             at += _up(math.prod(shape) * (4 if dtype == torch.float32 else 2))
         groups.append(group)
-    return groups, vec, vec2, at
+    return groups, (vec, vec2, again), at
 
 
 def plan_bytes(specs: Sequence[GroupSpec]) -> int:
-    return _layout(specs, choose_bn(specs))[3]
+    return _layout(specs, choose_bn(specs))[2]
 
 
 def _two_wide(e: np.ndarray) -> np.ndarray:
@@ -478,7 +479,7 @@ class Program:
         self.captured = False       # a CUDA graph names the lists
         self.bn = choose_bn(self.specs)
         self.wide = choose_wide(self.specs, self.bn)
-        self.groups, self.vec, self.vec2, self.nbytes = _layout(self.specs, self.bn)
+        self.groups, (self.vec, self.vec2, self.again), self.nbytes = _layout(self.specs, self.bn)
         self.n_matrices = sum(s.L for s in self.specs)
         assert self.n_matrices <= MAX_MATRICES
         self.first = [0]
@@ -569,6 +570,7 @@ class Plan:
         self.sumsq = arena.control[2 + n : 2 + 2 * n].view(torch.float32)
         self.vec = arena.at(program.vec, (n,), torch.float32)
         self.vec2 = arena.at(program.vec2, (n,), torch.float32)
+        self.again = arena.at(program.again, (n,), torch.int32)
         base = arena.buf.data_ptr()
         self._maps, maps_at = program.encode(base)
         a = _Args()

@@ -40,9 +40,12 @@ __device__ __forceinline__ float block_sum(float v) {
   }
 
 // ---------------------------------------------------------------- Muon prologue
-template <typename TG, typename TM, typename TX>
+// kAgain: the second pass of DmuonPrologueArgs::again.  Nearly always no slot asks for it; then a
+// block reads one word and leaves.
+template <typename TG, typename TM, typename TX, bool kAgain>
 __global__ void __launch_bounds__(kBlock) prologue_kernel(const DmuonPrologueArgs a) {
   const int t = blockIdx.y;
+  if (kAgain && a.again[a.slot[t]] == 0) return;
   const TG* g = reinterpret_cast<const TG*>(a.grad[t]);
   TM* m = reinterpret_cast<TM*>(a.mom[t]);
   TX* x = reinterpret_cast<TX*>(a.x[t]);
@@ -62,23 +65,24 @@ __global__ void __launch_bounds__(kBlock) prologue_kernel(const DmuonPrologueArg
     for (int k = 0; k < kVec; ++k) {
       const float gg = gv[k] * gs;
       // round the stored momentum first so that u uses what the next step will read
-      mv[k] = Conv<TM>::to(Conv<TM>::from(fmaf(mu, mv[k], gg)));
+      if (!kAgain) mv[k] = Conv<TM>::to(Conv<TM>::from(fmaf(mu, mv[k], gg)));
       uv[k] = a.nesterov ? fmaf(mu, mv[k], gg) : mv[k];
       acc = fmaf(uv[k], uv[k], acc);
       uv[k] *= xs;
     }
-    store8<TM>(m + i * kVec, mv);
+    if (!kAgain) store8<TM>(m + i * kVec, mv);
     store8<TX>(x + i * kVec, uv);
   }
   for (long long i = nvec * kVec + static_cast<long long>(blockIdx.x) * kBlock + threadIdx.x; i < n;
        i += stride) {
     const float gg = Conv<TG>::to(g[i]) * gs;
-    const TM mn = Conv<TM>::from(fmaf(mu, Conv<TM>::to(m[i]), gg));
-    m[i] = mn;
+    const TM mn = kAgain ? m[i] : Conv<TM>::from(fmaf(mu, Conv<TM>::to(m[i]), gg));
+    if (!kAgain) m[i] = mn;
     const float u = a.nesterov ? fmaf(mu, Conv<TM>::to(mn), gg) : Conv<TM>::to(mn);
     x[i] = Conv<TX>::from(u * xs);
     acc = fmaf(u, u, acc);
   }
+  if (kAgain) return;
   const float total = block_sum(acc);
   if (threadIdx.x == 0 && total != 0.f) atomicAdd(a.sumsq + a.slot[t], total);
 }
@@ -92,15 +96,27 @@ __global__ void norm_scales_kernel(const DmuonNormArgs a) {
   }
 }
 
+// How far this step's k / ||u|| may lie from the factor an operand was stored with.  Above: no entry of the
+// normalised matrix exceeds 1, so stored ones stay below 64 k, and so does what a restart stores; k is about
+// sqrt(min dimension), so that is 8192 of fp16's 65504 at a dimension of 14336.  Below: the entries' rms is at least
+// 1 / (64 * sqrt(max dimension)), 1.3e-4 at 14336, where half the spacing of fp16's subnormals (3e-8) is as much
+// against the rms as half an ulp of a normal number (2.4e-4): not less precise than right beside the norm.
+constexpr float kScaleRange = 64.f;
+
 __global__ void rescale_kernel(const DmuonRescaleArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < a.n) {
-    const float s = 1.f / (sqrtf(a.sumsq[i]) + a.eps);
-    const float k = a.k[i];
-    const float v = a.fresh ? 1.f / k : s / a.prescale[i];
+    const float norm = sqrtf(a.sumsq[i]) + a.eps;
+    const float s = 1.f / norm;
+    const float k = a.k[i], stored = a.prescale[i];
+    const float off = stored * norm / k;
+    // no factor yet (0), a matrix that was zero (1e7 k) or not finite before, a norm that jumped: not in the range
+    const bool good = off >= 1.f / kScaleRange && off <= kScaleRange;
+    const float v = good ? s / stored : 1.f / k;
     a.vec[i] = v;
     a.vec2[i] = v * v;
     a.prescale[i] = s * k;
+    a.again[i] = good ? 0 : 1;
   }
 }
 
@@ -262,7 +278,23 @@ extern "C" int dmuon_muon_prologue(const DmuonPrologueArgs* a, void* stream_v) {
   dim3 grid(blocks_per_tensor(a->n, a->numel), a->n);
   DMUON_DISPATCH(a->grad_dtype, TG,
     DMUON_DISPATCH(a->mom_dtype, TM,
-      DMUON_DISPATCH(a->x_dtype, TX, prologue_kernel<TG, TM, TX><<<grid, kBlock, 0, st>>>(*a))));
+      DMUON_DISPATCH(a->x_dtype, TX, prologue_kernel<TG, TM, TX, false><<<grid, kBlock, 0, st>>>(*a))));
+  count_launch();
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int dmuon_muon_prologue_again(const DmuonPrologueArgs* a, void* stream_v) {
+  if (a->n <= 0) return 0;
+  if (a->n > DMUON_MAX_TENSORS || a->again == nullptr || a->xscale == nullptr || a->x_dtype != DMUON_FP16) return -1;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
+  // Eight blocks an SM for one tensor, four for all of many: enough to stream at the memory's rate when a matrix
+  // has to be written again, few enough to be gone in no time when none has.
+  int bx = blocks_per_tensor(a->n, a->numel);
+  const int cap = a->n == 1 ? 148 * 8 : (148 * 4 + a->n - 1) / a->n;
+  if (bx > cap) bx = cap;
+  dim3 grid(bx, a->n);
+  DMUON_DISPATCH(a->grad_dtype, TG,
+    DMUON_DISPATCH(a->mom_dtype, TM, prologue_kernel<TG, TM, __half, true><<<grid, kBlock, 0, st>>>(*a)));
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

@@ -30,20 +30,24 @@ struct DmuonPrologueArgs {
   // optional per-slot multiplier applied to the STORED x only (x = cast(u * xscale[slot]); sumsq stays
   // the sum of u^2): lets a 16-bit operand be written in the same pass with a scale known beforehand
   const float* xscale;
+  // second pass over the same tensors (fp16 x only): where again[slot] != 0, x is written once more from the
+  // gradient and the momentum as updated, with the xscale of now; nothing else changes
+  const int* again;
 };
 
 // Scales of fp16 Gram operands that were stored with a factor known before the norm:
 //   s = 1 / (sqrt(sumsq) + eps);  vec = s / prescale (the products' correction), vec2 = vec^2,
 //   prescale = s * k (what the matrix is stored with next time)
-// fresh: the operand will be stored with the new prescale itself, so vec = 1 / k.
+// A factor from which this step's norm is too far (or none: 0) does not do: again[i] = 1 asks for the
+// operand to be stored with the new prescale itself, and vec = 1 / k.
 struct DmuonRescaleArgs {
   const float* sumsq;
   const float* k;
   float* prescale;
   float* vec;
   float* vec2;
+  int* again;
   int n;
-  int fresh;
   float eps;
 };
 
@@ -101,6 +105,7 @@ struct DmuonCastArgs {
 };
 
 int dmuon_muon_prologue(const DmuonPrologueArgs* a, void* stream);
+int dmuon_muon_prologue_again(const DmuonPrologueArgs* a, void* stream);
 int dmuon_norm_scales(const DmuonNormArgs* a, void* stream);
 int dmuon_rescale(const DmuonRescaleArgs* a, void* stream);
 int dmuon_adamw(const DmuonAdamWArgs* a, void* stream);

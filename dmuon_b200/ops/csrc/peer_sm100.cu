@@ -127,6 +127,8 @@ __global__ void __launch_bounds__(kBlock) peer_prologue_kernel(const DmuonPeerPr
     if (!block_wait_flags(a.ready_flags, 0, a.world, a.ready_want, a.budget_cycles, a.status)) return;
   }
   const int t = blockIdx.y;
+  const bool again = a.again != nullptr;
+  if (again && a.again[a.slot[t]] == 0) return;
   const long long off = a.offset[t];
   TM* m = reinterpret_cast<TM*>(a.mom[t]);
   TX* x = reinterpret_cast<TX*>(a.x[t]);
@@ -169,10 +171,10 @@ __global__ void __launch_bounds__(kBlock) peer_prologue_kernel(const DmuonPeerPr
 #pragma unroll
       for (int k = 0; k < kVec; ++k) {
         const float gg = sum[k] * gs;
-        mv[k] = Cv<TM>::to(Cv<TM>::from(fmaf(mu, mv[k], gg)));
+        if (!again) mv[k] = Cv<TM>::to(Cv<TM>::from(fmaf(mu, mv[k], gg)));
         uv[k] = a.nesterov ? fmaf(mu, mv[k], gg) : mv[k];
       }
-      st8<TM>(m + i * kVec, mv);
+      if (!again) st8<TM>(m + i * kVec, mv);
     } else {
 #pragma unroll
       for (int k = 0; k < kVec; ++k) uv[k] = sum[k] * gs;
@@ -191,13 +193,14 @@ __global__ void __launch_bounds__(kBlock) peer_prologue_kernel(const DmuonPeerPr
     const float gg = s * gs;
     float u = gg;
     if (m != nullptr) {
-      const TM mn = Cv<TM>::from(fmaf(mu, Cv<TM>::to(m[i]), gg));
-      m[i] = mn;
+      const TM mn = again ? m[i] : Cv<TM>::from(fmaf(mu, Cv<TM>::to(m[i]), gg));
+      if (!again) m[i] = mn;
       u = a.nesterov ? fmaf(mu, Cv<TM>::to(mn), gg) : Cv<TM>::to(mn);
     }
     x[i] = Cv<TX>::from(u * xs);
     acc = fmaf(u, u, acc);
   }
+  if (again) return;
   const float total = blk_sum(acc);
   if (threadIdx.x == 0 && a.sumsq != nullptr && !(total == 0.f)) atomicAdd(a.sumsq + a.slot[t], total);
 }

@@ -31,6 +31,8 @@ __device__ __forceinline__ float tp_block_sum(float v) {
 template <typename TG, typename TM, typename TX>
 __global__ void __launch_bounds__(kBlock) tp_gather_prologue_kernel(const DmuonTpGatherArgs a) {
   const int t = blockIdx.y;
+  const bool again = a.again != nullptr;
+  if (again && a.again[a.slot[t]] == 0) return;
   const TG* g = reinterpret_cast<const TG*>(a.src[t]);
   TM* m = reinterpret_cast<TM*>(a.mom[t]);
   TX* x = reinterpret_cast<TX*>(a.x[t]);
@@ -56,10 +58,10 @@ __global__ void __launch_bounds__(kBlock) tp_gather_prologue_kernel(const DmuonT
 #pragma unroll
         for (int k = 0; k < kVec; ++k) {
           const float gg = gv[k] * gs;
-          mv[k] = Conv<TM>::to(Conv<TM>::from(fmaf(mu, mv[k], gg)));
+          if (!again) mv[k] = Conv<TM>::to(Conv<TM>::from(fmaf(mu, mv[k], gg)));
           uv[k] = a.nesterov ? fmaf(mu, mv[k], gg) : mv[k];
         }
-        store8<TM>(m + d, mv);
+        if (!again) store8<TM>(m + d, mv);
       } else {
 #pragma unroll
         for (int k = 0; k < kVec; ++k) uv[k] = gv[k] * gs;
@@ -79,14 +81,15 @@ __global__ void __launch_bounds__(kBlock) tp_gather_prologue_kernel(const DmuonT
       const float gg = Conv<TG>::to(g[i]) * gs;
       float u = gg;
       if (m != nullptr) {
-        const TM mn = Conv<TM>::from(fmaf(mu, Conv<TM>::to(m[d]), gg));
-        m[d] = mn;
+        const TM mn = again ? m[d] : Conv<TM>::from(fmaf(mu, Conv<TM>::to(m[d]), gg));
+        if (!again) m[d] = mn;
         u = a.nesterov ? fmaf(mu, Conv<TM>::to(mn), gg) : Conv<TM>::to(mn);
       }
       x[d] = Conv<TX>::from(u * xs);
       acc = fmaf(u, u, acc);
     }
   }
+  if (again) return;
   const float total = tp_block_sum(acc);
   if (threadIdx.x == 0 && a.sumsq != nullptr && !(total == 0.f)) atomicAdd(a.sumsq + a.slot[t], total);
 }

@@ -44,6 +44,7 @@ struct DmuonTpGatherArgs {
   const float* gscale;
   float* sumsq;                       // may be null
   const float* xscale;                // may be null
+  const int* again;                   // may be null; second pass, see DmuonPrologueArgs
 };
 
 // For job t:  dst[t][r * cols + c] = dst * decay[t] + src[t][r * pitch + c]

@@ -27,6 +27,7 @@ class _PrologueArgs(ctypes.Structure):
         ("n", ctypes.c_int), ("grad_dtype", ctypes.c_int), ("mom_dtype", ctypes.c_int), ("x_dtype", ctypes.c_int),
         ("mu", ctypes.c_float), ("nesterov", ctypes.c_int),
         ("gscale", ctypes.c_void_p), ("sumsq", ctypes.c_void_p), ("xscale", ctypes.c_void_p),
+        ("again", ctypes.c_void_p),
     ]
 
 
@@ -65,8 +66,8 @@ class _CastArgs(ctypes.Structure):
 class _RescaleArgs(ctypes.Structure):
     _fields_ = [
         ("sumsq", ctypes.c_void_p), ("k", ctypes.c_void_p), ("prescale", ctypes.c_void_p),
-        ("vec", ctypes.c_void_p), ("vec2", ctypes.c_void_p),
-        ("n", ctypes.c_int), ("fresh", ctypes.c_int), ("eps", ctypes.c_float),
+        ("vec", ctypes.c_void_p), ("vec2", ctypes.c_void_p), ("again", ctypes.c_void_p),
+        ("n", ctypes.c_int), ("eps", ctypes.c_float),
     ]
 
 
@@ -75,6 +76,7 @@ def _lib():
     lib = _build.load()
     for name, typ in (
         ("dmuon_muon_prologue", _PrologueArgs),
+        ("dmuon_muon_prologue_again", _PrologueArgs),
         ("dmuon_norm_scales", _NormArgs),
         ("dmuon_rescale", _RescaleArgs),
         ("dmuon_adamw", _AdamWArgs),
@@ -123,15 +125,18 @@ def muon_prologue(
     nesterov: bool,
     gscale: Optional[torch.Tensor] = None,
     xscale: Optional[torch.Tensor] = None,
-) -> None:
+) -> list:
     """``mom = mu*mom + g``; ``u = g + mu*mom`` (or ``mom``); ``x = cast(u)``;
     accumulate ``sum(u^2)`` into ``sumsq[slot]`` (``sumsq`` must be zeroed by the
     caller).  With ``xscale`` (fp32, one entry per slot) the stored operand is
-    ``cast(u * xscale[slot])`` while the sum of squares stays that of ``u``."""
+    ``cast(u * xscale[slot])`` while the sum of squares stays that of ``u``.
+
+    Returns the argument blocks for :func:`muon_prologue_again`."""
     n = len(grads)
     assert n == len(moms) == len(xs) == len(slots)
+    blocks: list = []
     if n == 0:
-        return
+        return blocks
     dev = grads[0].device
     gd, md, xd = grads[0].dtype, moms[0].dtype, xs[0].dtype
     for lo, hi in _chunks(n):
@@ -151,6 +156,16 @@ def muon_prologue(
         a.sumsq = sumsq.data_ptr()
         a.xscale = xscale.data_ptr() if xscale is not None else None
         _check(_lib().dmuon_muon_prologue(ctypes.byref(a), _stream(dev)), "dmuon_muon_prologue")
+        blocks.append(a)
+    return blocks
+
+
+def muon_prologue_again(blocks: list, again: torch.Tensor) -> None:
+    """Second pass over the tensors of a :func:`muon_prologue` call with fp16 operands:
+    those with ``again[slot] != 0`` are stored once more, with the ``xscale`` of now."""
+    for a in blocks:
+        a.again = again.data_ptr()
+        _check(_lib().dmuon_muon_prologue_again(ctypes.byref(a), _stream(again.device)), "dmuon_muon_prologue_again")
 
 
 def norm_scales(sumsq: torch.Tensor, scale: torch.Tensor, scale2: torch.Tensor, eps: float = 1e-7) -> None:
@@ -162,14 +177,16 @@ def norm_scales(sumsq: torch.Tensor, scale: torch.Tensor, scale2: torch.Tensor, 
 
 def rescale(
     sumsq: torch.Tensor, k: torch.Tensor, prescale: torch.Tensor, vec: torch.Tensor, vec2: torch.Tensor,
-    fresh: bool, eps: float = 1e-7,
+    again: torch.Tensor, eps: float = 1e-7,
 ) -> None:
-    """Correction factors of operands that are stored times ``prescale`` (see the
-    argument block in ``csrc/multi_tensor.cuh``); ``prescale`` is updated in place."""
+    """Correction factors of operands that are stored times ``prescale`` (0: not known; see
+    the argument block in ``csrc/multi_tensor.cuh``); ``prescale`` is updated in place and
+    ``again`` (int32) says which operands have to be stored with the new one."""
     a = _RescaleArgs()
     a.sumsq, a.k, a.prescale = sumsq.data_ptr(), k.data_ptr(), prescale.data_ptr()
     a.vec, a.vec2 = vec.data_ptr(), vec2.data_ptr()
-    a.n, a.fresh, a.eps = sumsq.numel(), int(bool(fresh)), float(eps)
+    a.again = again.data_ptr()
+    a.n, a.eps = sumsq.numel(), float(eps)
     _check(_lib().dmuon_rescale(ctypes.byref(a), _stream(sumsq.device)), "dmuon_rescale")
 
 

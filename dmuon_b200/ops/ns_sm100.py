@@ -79,19 +79,23 @@ class _Workspace:
         self.scale = torch.empty(L, device=device, dtype=torch.float32)
         self.scale2 = torch.empty(L, device=device, dtype=torch.float32)
         self.Xf32: Optional[torch.Tensor] = None
-        # single-pass fp16 operand: the per-matrix correction factors of the current call
+        # single-pass fp16 operand: the per-matrix correction factors of the current call, whether an operand has to
+        # be stored once more, and the power of two in its scale
         self.fix = torch.empty(L, device=device, dtype=torch.float32)
         self.fix2 = torch.empty(L, device=device, dtype=torch.float32)
+        self.again = torch.empty(L, device=device, dtype=torch.int32)
+        self.k = torch.full((L,), CH.fp16_prescale(m0, n0), device=device, dtype=torch.float32)
 
     def nbytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in vars(self).values() if isinstance(t, torch.Tensor))
 
 
-#: fp16 Gram operands written by the prologue itself from the second step on (no fp32 staging pass);
+#: fp16 Gram operands written by the prologue itself (no fp32 staging pass);
 #: ``DMUON_NS_SINGLE_PASS=0`` keeps the two-pass form (norm first, then cast)
 SINGLE_PASS_FP16 = __import__("os").environ.get("DMUON_NS_SINGLE_PASS", "1").strip().lower() not in ("0", "false", "no", "off")
 
-#: per batch of matrices (keyed by their momentum buffers): K / ||u|| of their previous step
+#: per batch of matrices (keyed by their momentum buffers): K / ||u|| of their previous step.  A guess for this
+#: step's, checked on the device against the norm itself: a wrong one costs a second pass, not precision.
 _prescales: dict[tuple, torch.Tensor] = {}
 _workspaces: dict[tuple, _Workspace] = {}
 _ptr_tables: dict[tuple, torch.Tensor] = {}
@@ -472,30 +476,32 @@ def _has_publish(publish) -> bool:
     return publish is not None and all(p is not None for p in publish)
 
 
-def _muon_update_chain(plan: "CH.Plan", jobs: Sequence[UpdateJob]) -> None:
-    eps = 1e-7
-    moms = [m for j in jobs for m in j.moms]
-    owner_key = tuple(m.data_ptr() for m in moms)
-    pre = _prescales.get(owner_key)
-    fresh = pre is None
-    if fresh:
+def _prescale_of(moms: Sequence[torch.Tensor]) -> torch.Tensor:
+    """The stored factors of these matrices; zeros where none is known."""
+    key = tuple(m.data_ptr() for m in moms)
+    pre = _prescales.get(key)
+    if pre is None:
         if len(_prescales) > 4096:
             _prescales.clear()
-        pre = torch.empty_like(plan.vec)
+        pre = _prescales[key] = torch.zeros(len(moms), dtype=torch.float32, device=moms[0].device)
+    return pre
+
+
+def _muon_update_chain(plan: "CH.Plan", jobs: Sequence[UpdateJob]) -> None:
+    eps = 1e-7
+    pre = _prescale_of([m for j in jobs for m in j.moms])
     operands = [x for X in plan.X for x in X]
-    stage = [torch.empty(x.shape, dtype=torch.float32, device=x.device) for x in operands] if fresh else operands
     slots = range(plan.n_matrices)
     plan.begin()
     first = 0
+    blocks: list = []
     for j in jobs:
         n, o = len(j.moms), j.options
-        MT.muon_prologue(j.grads, j.moms, stage[first : first + n], slots[first : first + n], plan.sumsq, o["mu"],
-                         o["nesterov"], o["gscale"], xscale=None if fresh else pre)
+        blocks += MT.muon_prologue(j.grads, j.moms, operands[first : first + n], slots[first : first + n], plan.sumsq,
+                                   o["mu"], o["nesterov"], o["gscale"], xscale=pre)
         first += n
-    MT.rescale(plan.sumsq, plan.k, pre, plan.vec, plan.vec2, fresh, eps)
-    if fresh:
-        MT.cast(stage, operands, scale=pre, slots=slots)
-        _prescales[owner_key] = pre
+    MT.rescale(plan.sumsq, plan.k, pre, plan.vec, plan.vec2, plan.again, eps)
+    MT.muon_prologue_again(blocks, plan.again)
     finals = []
     for j in jobs:
         o = j.options
@@ -554,12 +560,13 @@ def muon_update_batched(
         return False
     m0, n0 = int(moms[0].shape[0]), int(moms[0].numel() // moms[0].shape[0])
     dev = moms[0].device
+    blocks: list = []
 
-    def prologue(xs_out, xscale=None):
+    def prologue(xs_out, xscale=None, again=None):
         if peer is not None and hasattr(peer, "launch_prologue"):
             # tensor-parallel gather fused into the prologue: every shard is read where it lies
             peer.launch_prologue(moms, xs_out, slots, ws.sumsq, mu=mu, nesterov=nesterov, gscale=gscale,
-                                 xscale=xscale)
+                                 xscale=xscale, again=again)
         elif peer is not None:
             # reduce-to-owner fused into the prologue: gradients are read from
             # every rank's arena through its peer mapping
@@ -568,33 +575,33 @@ def muon_update_batched(
             P.peer_prologue(peer.peer_bases, peer.offsets, peer.numels, peer.grad_dtype, moms, xs_out, slots,
                             ws.sumsq, scale=peer.scale, mu=mu, nesterov=nesterov, gscale=gscale,
                             ready_flags=peer.ready_flags, ready_want=peer.ready_want, status=peer.status,
-                            xscale=xscale)
+                            xscale=xscale, again=again)
+        elif again is not None:
+            MT.muon_prologue_again(blocks, again)
         else:
-            MT.muon_prologue(grads, moms, xs_out, slots, ws.sumsq, mu, nesterov, gscale, xscale=xscale)
+            blocks.extend(MT.muon_prologue(grads, moms, xs_out, slots, ws.sumsq, mu, nesterov, gscale, xscale=xscale))
 
     cd = _resolve_dtype(compute_dtype, formulation)
     ws = workspace(L, m0, n0, cd, dev)
     left = m0 <= n0
     ws.sumsq.zero_()
     slots = list(range(L))
-    owner_key = tuple(m.data_ptr() for m in moms)     # which matrices: their momentum buffers live as long as they do
     if cd == torch.bfloat16 and formulation == "gram":
         # one pass: the raw bf16 operand carries its scale as a per-matrix vector
         prologue([ws.X[i].reshape(-1) for i in range(L)])
         MT.norm_scales(ws.sumsq, ws.scale, ws.scale2, eps)
         xscale = _XScale(vec=ws.scale, vec2=ws.scale2)
-    elif cd == torch.float16 and formulation == "gram" and SINGLE_PASS_FP16 and owner_key in _prescales:
+    elif cd == torch.float16 and formulation == "gram" and SINGLE_PASS_FP16:
         # one pass: the fp16 operand is stored with LAST step's K / ||u|| of the same matrices (momentum
-        # makes the norm drift slowly, and fp16 has three orders of magnitude of room on either side of
-        # the entries' size), and the products carry the exact correction ||u||_prev / ||u||_now per
-        # matrix, so the result is scaled by this step's true norm
-        K = fp16_prescale(m0, n0)
-        pre = _prescales[owner_key]
-        prologue([ws.X[i].reshape(-1) for i in range(L)], xscale=pre)
-        MT.norm_scales(ws.sumsq, ws.scale, ws.scale2, eps)
-        torch.div(ws.scale, pre, out=ws.fix)                  # (1/||u||) / (K/||u||_prev)
-        torch.mul(ws.fix, ws.fix, out=ws.fix2)
-        torch.mul(ws.scale, K, out=pre)                       # what the next step stores with
+        # makes the norm drift slowly, and fp16 has room on either side of the entries' size), and the
+        # products carry the exact correction ||u||_prev / ||u||_now per matrix, so the result is scaled by
+        # this step's true norm.  Where that factor is too far off, or not known, the operand is stored once
+        # more with this step's (`again`): the peers' gradients are still there, they are handed back after the step.
+        pre = _prescale_of(moms)
+        operands = [ws.X[i].reshape(-1) for i in range(L)]
+        prologue(operands, xscale=pre)
+        MT.rescale(ws.sumsq, ws.k, pre, ws.fix, ws.fix2, ws.again, eps)
+        prologue(operands, xscale=pre, again=ws.again)
         xscale = _XScale(vec=ws.fix, vec2=ws.fix2)
     else:
         # two passes: fp32 staging, then normalise (and prescale fp16) while casting
@@ -608,11 +615,6 @@ def muon_update_batched(
             ws.scale.mul_(K)
         MT.cast(stage, [ws.X[i] for i in range(L)], scale=ws.scale, slots=slots)
         xscale = _XScale(h=1.0 / K)
-        if cd == torch.float16 and formulation == "gram" and SINGLE_PASS_FP16:
-            # from the next step on these matrices take the single-pass path (ws.scale holds K / ||u||)
-            if len(_prescales) > 4096:
-                _prescales.clear()
-            _prescales[owner_key] = ws.scale.clone()
 
     step_alpha = -float(lr) * float(update_scale)
     if formulation == "direct":

@@ -37,6 +37,7 @@ class _PeerPrologueArgs(ctypes.Structure):
         ("mu", ctypes.c_float), ("nesterov", ctypes.c_int), ("gscale", ctypes.c_void_p), ("sumsq", ctypes.c_void_p),
         ("ready_flags", ctypes.c_void_p), ("ready_want", ctypes.c_int), ("budget_cycles", ctypes.c_longlong),
         ("status", ctypes.c_void_p), ("max_blocks_per_tensor", ctypes.c_int), ("xscale", ctypes.c_void_p),
+        ("again", ctypes.c_void_p),
     ]
 
 
@@ -170,11 +171,14 @@ def peer_prologue(
     budget_cycles: Optional[int] = None,
     max_blocks_per_tensor: int = 0,
     xscale: Optional[torch.Tensor] = None,
+    again: Optional[torch.Tensor] = None,
 ) -> None:
     """Sum the gradient of every listed tensor over all ranks' arenas (peer
     loads, rank order), scale, then momentum / Nesterov / cast / sum of squares
     exactly like :func:`multi_tensor.muon_prologue`.  ``moms[i] is None`` turns
-    the momentum off for that launch (all entries of one call must agree)."""
+    the momentum off for that launch (all entries of one call must agree).  With
+    ``again`` (int32 per slot) this is the second pass over the same tensors: where it is
+    set, ``xs`` is stored once more with the ``xscale`` of now, nothing else changes."""
     n = len(offsets)
     if n == 0:
         return
@@ -204,6 +208,7 @@ def peer_prologue(
         a.status = status.data_ptr() if status is not None else None
         a.max_blocks_per_tensor = int(max_blocks_per_tensor)
         a.xscale = xscale.data_ptr() if xscale is not None else None
+        a.again = again.data_ptr() if again is not None else None
         _check(_lib().dmuon_peer_prologue(ctypes.byref(a), _stream(dev)), "dmuon_peer_prologue")
 
 

@@ -22,7 +22,7 @@ class _GatherArgs(ctypes.Structure):
         ("src", _VP), ("mom", _VP), ("x", _VP), ("rows", _IA), ("cols", _IA), ("pitch", _LL), ("slot", _IA),
         ("n", ctypes.c_int), ("src_dtype", ctypes.c_int), ("mom_dtype", ctypes.c_int), ("x_dtype", ctypes.c_int),
         ("mu", ctypes.c_float), ("nesterov", ctypes.c_int), ("gscale", ctypes.c_void_p), ("sumsq", ctypes.c_void_p),
-        ("xscale", ctypes.c_void_p),
+        ("xscale", ctypes.c_void_p), ("again", ctypes.c_void_p),
     ]
 
 
@@ -68,13 +68,15 @@ def gather_prologue(
     nesterov: bool,
     gscale: Optional[torch.Tensor] = None,
     xscale: Optional[torch.Tensor] = None,
+    again: Optional[torch.Tensor] = None,
 ) -> None:
     """Momentum / Nesterov / cast / sum of squares of full matrices whose
     gradient arrives as shards (``jobs``): every shard is read where it lies --
     on this GPU or, through its peer mapping, on another one -- and written into
     the rows / columns it occupies in ``moms[i]`` and ``xs[i]`` (full matrices,
     row-major, contiguous).  ``moms[i] is None`` for all ``i`` switches the
-    momentum off (``x = cast(g)``)."""
+    momentum off (``x = cast(g)``).  ``again``: the second pass, as in
+    :func:`dmuon_b200.ops.peer.peer_prologue`."""
     if not jobs:
         return
     dev = xs[0].device
@@ -99,6 +101,7 @@ def gather_prologue(
         a.gscale = gscale.data_ptr() if gscale is not None else None
         a.sumsq = sumsq.data_ptr() if sumsq is not None else None
         a.xscale = xscale.data_ptr() if xscale is not None else None
+        a.again = again.data_ptr() if again is not None else None
         _check(_lib().dmuon_tp_gather_prologue(ctypes.byref(a), _stream(dev)), "dmuon_tp_gather_prologue")
 
 

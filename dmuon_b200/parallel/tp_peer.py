@@ -92,9 +92,10 @@ class TPGatherSource:
         self.sources = sources
         self.exchange = sources[0].exchange
 
-    def launch_prologue(self, moms, xs_out, slots, sumsq, *, mu, nesterov, gscale=None, xscale=None) -> None:
+    def launch_prologue(self, moms, xs_out, slots, sumsq, *, mu, nesterov, gscale=None, xscale=None,
+                        again=None) -> None:
         self.exchange.gather_prologue([s.dparam for s in self.sources], moms, xs_out, slots, sumsq, mu=mu,
-                                      nesterov=nesterov, gscale=gscale, xscale=xscale)
+                                      nesterov=nesterov, gscale=gscale, xscale=xscale, again=again)
 
 
 class TPPeerExchange:
@@ -212,7 +213,8 @@ class TPPeerExchange:
                                      r_off * cols + c_off, cols))
         return jobs
 
-    def gather_prologue(self, dparams, moms, xs_out, slots, sumsq, *, mu, nesterov, gscale=None, xscale=None) -> None:
+    def gather_prologue(self, dparams, moms, xs_out, slots, sumsq, *, mu, nesterov, gscale=None, xscale=None,
+                        again=None) -> None:
         """Prologue of full matrices whose gradient shards are read from the
         ranks of the group (bounded wait for their "ready" flags first)."""
         from ..ops import tp_peer as K
@@ -220,7 +222,7 @@ class TPPeerExchange:
         with record_function(f"dmuon.tp_peer.gather_prologue.params{len(dparams)}"):
             self._wait_all(KIND_GRAD_READY, self.gather_epoch)
             K.gather_prologue(self._jobs(dparams), self.grad_dtype, moms, xs_out, slots, sumsq, mu=mu,
-                              nesterov=nesterov, gscale=gscale, xscale=xscale)
+                              nesterov=nesterov, gscale=gscale, xscale=xscale, again=again)
 
     def materialize(self, p) -> torch.Tensor:
         out = torch.empty(p.full_shape, dtype=torch.float32, device=self.device)

@@ -214,3 +214,86 @@ def test_replays_beside_eager_calls_on_other_streams():
     G.check_status(dev)
     for out, w in got:
         assert _rel(out, w.double()) < 1e-2
+
+
+class _LocalPeer:
+    """The gradients of a batch as the peer plane hands them over, all on this GPU."""
+
+    def __init__(self, grads):
+        self.keep = torch.cat([g.reshape(-1) for g in grads])
+        self.peer_bases, self.grad_dtype, self.scale = [self.keep.data_ptr()], self.keep.dtype, 1.0
+        self.numels = [g.numel() for g in grads]
+        self.offsets = [sum(self.numels[:i]) for i in range(len(grads))]
+        self.ready_flags, self.ready_want, self.status = None, 0, None
+
+
+class _LocalShards:
+    """The gradients of a batch as tensor-parallel shards (halves of the rows), all on this GPU."""
+
+    def __init__(self, grads):
+        self.shards = [[s.contiguous() for s in g.chunk(2)] for g in grads]
+
+    def launch_prologue(self, moms, xs, slots, sumsq, **kw):
+        from dmuon_b200.ops import tp_peer as TP
+
+        jobs = []
+        for i, pair in enumerate(self.shards):
+            row = 0
+            for s in pair:
+                jobs.append(TP.ShardJob(i, s.data_ptr(), s.shape[0], s.shape[1], row * s.shape[1], s.shape[1]))
+                row += s.shape[0]
+        TP.gather_prologue(jobs, self.shards[0][0].dtype, moms, xs, slots, sumsq, **kw)
+
+
+@pytest.mark.parametrize("form", ["chain", "launches", "peer", "shards"])
+@pytest.mark.parametrize("mom_dtype", [torch.float32, torch.bfloat16])
+def test_update_after_zero_and_jumping_gradients(form, mom_dtype, monkeypatch):
+    """The factor that an fp16 operand is stored with is last step's; steps after which it does not do."""
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+
+    if form != "chain":
+        monkeypatch.setattr(ns_sm100, "_chain_pays", lambda specs: False)
+    dev = _dev()
+    torch.manual_seed(12)
+    shapes = [(3, 264, 1024), (2, 1032, 256)]
+    coefs, restarts, lr, wd, mu = list(NS.DEFAULT_COEFFICIENTS), [2], 0.02, 0.1, 0.9
+    moms = [[torch.zeros(m, n, device=dev, dtype=mom_dtype) for _ in range(L)] for L, m, n in shapes]
+    masters = [[torch.randn(m, n, device=dev) * 0.02 for _ in range(L)] for L, m, n in shapes]
+    # magnitudes of the gradients, whether the momentum starts from zero: no gradient at all, a norm 1e5 times as large,
+    # one 1e10 times smaller, 50 times either way (inside the range of a stored factor), zero again
+    for step, (mag, zero) in enumerate([(0.0, False), (1e-3, False), (1e2, False), (1e-8, True), (5e-7, True),
+                                        (1e-8, True), (0.0, True), (1e-2, False), (1e-2, False)]):
+        grads = [[(torch.randn(m, n, device=dev) * mag).bfloat16() for _ in range(L)] for L, m, n in shapes]
+        if step == 4:
+            grads[0][1].zero_()               # one matrix of a batch
+        if zero:
+            for x in (*moms[0], *moms[1]):
+                x.zero_()
+        m_prev = [[x.clone() for x in g] for g in moms]
+        w_prev = [[x.clone() for x in g] for g in masters]
+        jobs = []
+        for g, (L, m, n) in enumerate(shapes):
+            peer = {"peer": _LocalPeer, "shards": _LocalShards}.get(form, lambda grads: None)(grads[g])
+            options = dict(mu=mu, nesterov=True, coefs=coefs, restarts=restarts, formulation="gram", lr=lr,
+                           weight_decay=wd, update_scale=0.2 * math.sqrt(max(m, n)), compute_dtype=None, gscale=None,
+                           peer=peer)
+            jobs.append(ns_sm100.UpdateJob(grads[g] if peer is None else None, moms[g], masters[g], options))
+        ns_sm100.muon_update_groups(jobs, lambda i, wrote: None)
+        torch.cuda.synchronize()
+        G.check_status(dev)
+        for g, (L, m, n) in enumerate(shapes):
+            for i in range(L):
+                buf = (mu * m_prev[g][i].float() + grads[g][i].float()).to(mom_dtype).float()
+                u = grads[g][i].float() + mu * buf
+                o = NS.gram_newton_schulz(u, coefficients=coefs, restart_iterations=restarts, deterministic=True,
+                                          compute_dtype=torch.float32)
+                delta = masters[g][i] - w_prev[g][i] * (1 - lr * wd)
+                want = -lr * 0.2 * math.sqrt(max(m, n)) * o
+                # one rounding here, two in the kernel's fused form
+                ulp = 1e-2 if mom_dtype == torch.bfloat16 else 1e-6
+                assert torch.allclose(moms[g][i].float(), buf, rtol=ulp, atol=ulp * float(buf.abs().max()))
+                # fp16 products on well conditioned matrices, 0.005 seen; a result of zeros leaves the rounding of the
+                # weight itself (6e-8 of 0.02)
+                assert (delta - want).norm() < 1.5e-2 * want.norm() + 1e-8 * math.sqrt(m * n), (step, g, i)
