@@ -104,18 +104,20 @@ __global__ void norm_scales_kernel(const DmuonNormArgs a) {
 constexpr float kScaleRange = 64.f;
 
 __global__ void rescale_kernel(const DmuonRescaleArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < a.n) {
+  const int g = blockIdx.y;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = a.first[g] + j;
+  if (i < a.first[g + 1]) {
     const float norm = sqrtf(a.sumsq[i]) + a.eps;
     const float s = 1.f / norm;
-    const float k = a.k[i], stored = a.prescale[i];
+    const float k = a.k[i], stored = a.prescale[g][j];
     const float off = stored * norm / k;
     // no factor yet (0), a matrix that was zero (1e7 k) or not finite before, a norm that jumped: not in the range
     const bool good = off >= 1.f / kScaleRange && off <= kScaleRange;
     const float v = good ? s / stored : 1.f / k;
     a.vec[i] = v;
     a.vec2[i] = v * v;
-    a.prescale[i] = s * k;
+    a.prescale[g][j] = s * k;
     a.again[i] = good ? 0 : 1;
   }
 }
@@ -308,9 +310,16 @@ extern "C" int dmuon_norm_scales(const DmuonNormArgs* a, void* stream_v) {
 }
 
 extern "C" int dmuon_rescale(const DmuonRescaleArgs* a, void* stream_v) {
-  if (a->n <= 0) return 0;
+  if (a->groups <= 0) return 0;
+  if (a->groups > DMUON_MAX_RESCALE_GROUPS) return -1;
+  int most = 1;
+  for (int g = 0; g < a->groups; ++g) {
+    const int n = a->first[g + 1] - a->first[g];
+    if (n < 0 || (n > 0 && a->prescale[g] == nullptr)) return -1;
+    most = n > most ? n : most;
+  }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
-  rescale_kernel<<<(a->n + 127) / 128, 128, 0, st>>>(*a);
+  rescale_kernel<<<dim3((most + 127) / 128, a->groups), 128, 0, st>>>(*a);
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }

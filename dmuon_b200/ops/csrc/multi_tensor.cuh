@@ -20,7 +20,7 @@ struct DmuonPrologueArgs {
   void* mom[DMUON_MAX_TENSORS];
   void* x[DMUON_MAX_TENSORS];
   long long numel[DMUON_MAX_TENSORS];
-  int slot[DMUON_MAX_TENSORS];   // index into sumsq
+  int slot[DMUON_MAX_TENSORS];   // index into sumsq, xscale and again
   int n;
   int grad_dtype, mom_dtype, x_dtype;
   float mu;
@@ -40,14 +40,17 @@ struct DmuonPrologueArgs {
 //   prescale = s * k (what the matrix is stored with next time)
 // A factor from which this step's norm is too far (or none: 0) does not do: again[i] = 1 asks for the
 // operand to be stored with the new prescale itself, and vec = 1 / k.
+// The prescales are kept per group: group g's matrices are first[g] .. first[g + 1] - 1 of the others.
+enum { DMUON_MAX_RESCALE_GROUPS = 16 };
 struct DmuonRescaleArgs {
   const float* sumsq;
   const float* k;
-  float* prescale;
+  float* prescale[DMUON_MAX_RESCALE_GROUPS];
+  int first[DMUON_MAX_RESCALE_GROUPS + 1];
+  int groups;
   float* vec;
   float* vec2;
   int* again;
-  int n;
   float eps;
 };
 

@@ -14,6 +14,7 @@ import torch
 from . import build as _build
 
 MAX_TENSORS = 48
+MAX_RESCALE_GROUPS = 16
 _DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 _VP = ctypes.c_void_p * MAX_TENSORS
 _LL = ctypes.c_longlong * MAX_TENSORS
@@ -65,9 +66,9 @@ class _CastArgs(ctypes.Structure):
 
 class _RescaleArgs(ctypes.Structure):
     _fields_ = [
-        ("sumsq", ctypes.c_void_p), ("k", ctypes.c_void_p), ("prescale", ctypes.c_void_p),
-        ("vec", ctypes.c_void_p), ("vec2", ctypes.c_void_p), ("again", ctypes.c_void_p),
-        ("n", ctypes.c_int), ("eps", ctypes.c_float),
+        ("sumsq", ctypes.c_void_p), ("k", ctypes.c_void_p), ("prescale", ctypes.c_void_p * MAX_RESCALE_GROUPS),
+        ("first", ctypes.c_int * (MAX_RESCALE_GROUPS + 1)), ("groups", ctypes.c_int),
+        ("vec", ctypes.c_void_p), ("vec2", ctypes.c_void_p), ("again", ctypes.c_void_p), ("eps", ctypes.c_float),
     ]
 
 
@@ -176,17 +177,21 @@ def norm_scales(sumsq: torch.Tensor, scale: torch.Tensor, scale2: torch.Tensor, 
 
 
 def rescale(
-    sumsq: torch.Tensor, k: torch.Tensor, prescale: torch.Tensor, vec: torch.Tensor, vec2: torch.Tensor,
+    sumsq: torch.Tensor, k: torch.Tensor, prescales: Sequence[torch.Tensor], vec: torch.Tensor, vec2: torch.Tensor,
     again: torch.Tensor, eps: float = 1e-7,
 ) -> None:
-    """Correction factors of operands that are stored times ``prescale`` (0: not known; see
-    the argument block in ``csrc/multi_tensor.cuh``); ``prescale`` is updated in place and
-    ``again`` (int32) says which operands have to be stored with the new one."""
+    """Correction factors of operands that are stored times their group's ``prescales`` (0:
+    not known; see the argument block in ``csrc/multi_tensor.cuh``), which are updated in
+    place; ``again`` (int32) says which operands have to be stored with the new one."""
+    assert len(prescales) <= MAX_RESCALE_GROUPS
     a = _RescaleArgs()
-    a.sumsq, a.k, a.prescale = sumsq.data_ptr(), k.data_ptr(), prescale.data_ptr()
+    a.sumsq, a.k, a.groups = sumsq.data_ptr(), k.data_ptr(), len(prescales)
+    for g, p in enumerate(prescales):
+        a.prescale[g], a.first[g + 1] = p.data_ptr(), a.first[g] + p.numel()
+    assert a.first[len(prescales)] == sumsq.numel()
     a.vec, a.vec2 = vec.data_ptr(), vec2.data_ptr()
     a.again = again.data_ptr()
-    a.n, a.eps = sumsq.numel(), float(eps)
+    a.eps = float(eps)
     _check(_lib().dmuon_rescale(ctypes.byref(a), _stream(sumsq.device)), "dmuon_rescale")
 
 

@@ -489,19 +489,18 @@ def _prescale_of(moms: Sequence[torch.Tensor]) -> torch.Tensor:
 
 def _muon_update_chain(plan: "CH.Plan", jobs: Sequence[UpdateJob]) -> None:
     eps = 1e-7
-    pre = _prescale_of([m for j in jobs for m in j.moms])
-    operands = [x for X in plan.X for x in X]
-    slots = range(plan.n_matrices)
+    # per job, so that a matrix without a gradient in this step changes its own shape's batch only
+    prescales = [_prescale_of(j.moms) for j in jobs]
     plan.begin()
-    first = 0
-    blocks: list = []
-    for j in jobs:
+    passes: list = []
+    for j, X, pre, lo in zip(jobs, plan.X, prescales, plan.program.first):
         n, o = len(j.moms), j.options
-        blocks += MT.muon_prologue(j.grads, j.moms, operands[first : first + n], slots[first : first + n], plan.sumsq,
-                                   o["mu"], o["nesterov"], o["gscale"], xscale=pre)
-        first += n
-    MT.rescale(plan.sumsq, plan.k, pre, plan.vec, plan.vec2, plan.again, eps)
-    MT.muon_prologue_again(blocks, plan.again)
+        blocks = MT.muon_prologue(j.grads, j.moms, list(X), range(n), plan.sumsq[lo : lo + n], o["mu"], o["nesterov"],
+                                  o["gscale"], xscale=pre)
+        passes.append((blocks, plan.again[lo : lo + n]))
+    MT.rescale(plan.sumsq, plan.k, prescales, plan.vec, plan.vec2, plan.again, eps)
+    for blocks, again in passes:
+        MT.muon_prologue_again(blocks, again)
     finals = []
     for j in jobs:
         o = j.options
@@ -600,7 +599,7 @@ def muon_update_batched(
         pre = _prescale_of(moms)
         operands = [ws.X[i].reshape(-1) for i in range(L)]
         prologue(operands, xscale=pre)
-        MT.rescale(ws.sumsq, ws.k, pre, ws.fix, ws.fix2, ws.again, eps)
+        MT.rescale(ws.sumsq, ws.k, [pre], ws.fix, ws.fix2, ws.again, eps)
         prologue(operands, xscale=pre, again=ws.again)
         xscale = _XScale(vec=ws.fix, vec2=ws.fix2)
     else:

@@ -297,3 +297,47 @@ def test_update_after_zero_and_jumping_gradients(form, mom_dtype, monkeypatch):
                 # fp16 products on well conditioned matrices, 0.005 seen; a result of zeros leaves the rounding of the
                 # weight itself (6e-8 of 0.02)
                 assert (delta - want).norm() < 1.5e-2 * want.norm() + 1e-8 * math.sqrt(m * n), (step, g, i)
+
+
+def test_update_with_changing_participation():
+    """A matrix without a gradient in a step: the others' stored factors serve on, all results stay right."""
+    from dmuon_b200.ops import chain as CH
+    from dmuon_b200.ops import gemm as G
+    from dmuon_b200.ops import ns_sm100
+    from dmuon_b200.optim import newton_schulz as NS
+
+    dev = _dev()
+    torch.manual_seed(13)
+    shapes = [(4, 136, 520), (2, 264, 1024), (2, 520, 136)]
+    coefs, restarts, lr, mu = list(NS.DEFAULT_COEFFICIENTS), [2], 0.02, 0.9
+    moms = [[torch.zeros(m, n, device=dev) for _ in range(L)] for L, m, n in shapes]
+    masters = [[torch.randn(m, n, device=dev) * 0.02 for _ in range(L)] for L, m, n in shapes]
+    CH.release()
+    for step, idle in enumerate([(), (2,), (), (0, 3), (2,), ()]):
+        here = [[i for i in range(L) if g or i not in idle] for g, (L, _, _) in enumerate(shapes)]
+        grads = [[(torch.randn(m, n, device=dev) * 1e-3).bfloat16() for _ in range(L)] for L, m, n in shapes]
+        m_prev = [[x.clone() for x in g] for g in moms]
+        w_prev = [[x.clone() for x in g] for g in masters]
+        jobs = []
+        for g, (L, m, n) in enumerate(shapes):
+            options = dict(mu=mu, nesterov=True, coefs=coefs, restarts=restarts, formulation="gram", lr=lr,
+                           weight_decay=0.0, update_scale=1.0, compute_dtype=None, gscale=None, peer=None)
+            pick = lambda ts: [ts[i] for i in here[g]]
+            jobs.append(ns_sm100.UpdateJob(pick(grads[g]), pick(moms[g]), pick(masters[g]), options))
+        ns_sm100.muon_update_groups(jobs, lambda i, wrote: None)
+        torch.cuda.synchronize()
+        G.check_status(dev)
+        plan = next(reversed(CH._plans.values()))
+        assert plan.n_matrices == sum(map(len, here))
+        if step:
+            assert not plan.again[len(here[0]):].any()
+        for g, (L, m, n) in enumerate(shapes):
+            for i in range(L):
+                if i not in here[g]:
+                    assert torch.equal(masters[g][i], w_prev[g][i]) and torch.equal(moms[g][i], m_prev[g][i])
+                    continue
+                u = grads[g][i].float() + mu * moms[g][i]
+                o = NS.gram_newton_schulz(u, coefficients=coefs, restart_iterations=restarts, deterministic=True,
+                                          compute_dtype=torch.float32)
+                # as above: fp16 products on well conditioned matrices
+                assert _rel(masters[g][i] - w_prev[g][i], -lr * o.double()) < 1.5e-2, (step, g, i)
