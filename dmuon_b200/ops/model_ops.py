@@ -244,13 +244,14 @@ class _LinearXent(torch.autograd.Function):
         saved = ctx.saved_tensors
         grads = [t for t in saved if t is not None]
         if grads:
-            # They are the results themselves, so they are scaled where they lie, unless this graph is kept
-            # and may be walked again.
             scale = g.to(grads[0].dtype)
-            if torch._C._autograd._get_current_graph_task_keep_graph() or torch.is_grad_enabled():
-                grads = torch._foreach_mul(grads, scale)
+            ft = torch._C._functorch
+            if torch.is_grad_enabled() or ft.is_legacy_batchedtensor(g) or ft.is_functorch_wrapped_tensor(g):
+                # second derivatives and batched walks: the list form has no rules for them
+                grads = [t * scale for t in grads]
             else:
-                torch._foreach_mul_(grads, scale)
+                # into new tensors: whoever packed the saved ones may hold them still
+                grads = torch._foreach_mul(grads, scale)
         it = iter(grads)
         d_h, d_w = (next(it) if t is not None else None for t in saved)
         return d_h, d_w, None, None, None
