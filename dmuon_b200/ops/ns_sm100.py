@@ -420,6 +420,7 @@ class UpdateJob:
     publish: Optional[Sequence[Optional[torch.Tensor]]] = None
     deltas: Optional[Sequence[torch.Tensor]] = None
     publish_multicast: Optional[Sequence[int]] = None
+    apart: bool = False         # the caller communicates the result: a launch of its own, issued in order
 
     @cached_property
     def spec(self) -> CH.GroupSpec:
@@ -439,11 +440,17 @@ class UpdateJob:
 
 
 def muon_update_groups(jobs: Sequence[UpdateJob], on_issued) -> None:
-    """:func:`muon_update_batched` for several shape groups.  Groups that are too small
-    to fill the GPU run side by side in shared launches of the product-chain kernel.
-    ``on_issued(i, wrote)`` is called as soon as the kernels of job ``i`` are issued
-    (``wrote`` as returned by :func:`muon_update_batched`), not after all jobs: callers
-    start communication there."""
+    """:func:`muon_update_batched` for several shape groups.  Groups share launches of the
+    product-chain kernel as far as one plan holds them, so that tiles of one fill the last
+    round of another.  Update of decoder layers on a B200, shared / a launch per shape:
+    four layers 1024 wide 1.02 / 1.43 ms, one 3072 wide 3.7 / 4.5, one 4096 wide 9.6 / 10.6;
+    where every shape has several rounds of its own it is a draw (sixteen layers 1024 wide
+    4.5 / 4.4, four 3072 wide 16.0 / 16.2, two 4096 wide 19.6 / 19.9).
+
+    ``on_issued(i, wrote)`` is called once the kernels of job ``i`` are issued (``wrote`` as
+    returned by :func:`muon_update_batched`); jobs of one launch are issued together.  A job
+    that is ``apart`` has a launch of its own and its callback comes before the next launch:
+    the caller's communication then runs beside it."""
 
     def alone(i: int) -> None:
         job = jobs[i]
@@ -454,7 +461,8 @@ def muon_update_groups(jobs: Sequence[UpdateJob], on_issued) -> None:
     for i, job in enumerate(jobs):
         if not job.moms or not job.chainable():
             alone(i)
-        elif chunks and _chain_pays([*(jobs[k].spec for k in chunks[-1]), job.spec]):
+        elif chunks and not job.apart and not jobs[chunks[-1][0]].apart \
+                and _chain_pays([*(jobs[k].spec for k in chunks[-1]), job.spec]):
             chunks[-1].append(i)
         else:
             chunks.append([i])

@@ -902,9 +902,10 @@ class Muon(torch.optim.Optimizer):
                             multicast = [rt.pub_mc + dp._arena_offset * esz for dp, _ in chunk]
                         else:
                             publish = [None] * len(chunk)       # published (cast + multicast) after the step
+                    replicate = nvls and multicast is None
                     jobs.append(ns_sm100.UpdateJob(grads, moms, masters, common, publish=publish,
-                                                   publish_multicast=multicast))
-                    after.append((chunk, nvls and multicast is None))
+                                                   publish_multicast=multicast, apart=replicate))
+                    after.append((chunk, replicate))
 
         def issued(i: int, wrote: bool) -> None:
             job, (chunk, replicate) = jobs[i], after[i]
@@ -914,7 +915,7 @@ class Muon(torch.optim.Optimizer):
                 return
             if replicate and wrote:
                 # the last product wrote the local slots: replicate them to all ranks on the
-                # publish lane while the next batch is orthogonalised
+                # publish lane while the next batch (a launch of its own) is orthogonalised
                 rt.multicast_publish_async([dp for dp, _ in chunk])
             for dp, _ in chunk:
                 dp._publish_fresh = bool(wrote)

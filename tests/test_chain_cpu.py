@@ -207,3 +207,23 @@ def test_capture_without_an_earlier_call_has_no_plan(streams):
     streams["capturing"] = True
     assert CH.plan_for([_spec(1, 64, 128)], torch.device("cuda", 0)) is None
     assert not CH._programs
+
+
+def test_jobs_whose_results_are_sent_have_launches_of_their_own(monkeypatch):
+    """... and their callback comes before the next launch; the others share one."""
+    import contextlib
+
+    from dmuon_b200.ops import ns_sm100
+
+    def job(m, n, apart):
+        options = dict(coefs=COEFS, restarts=(2,), formulation="gram", compute_dtype=None, peer=None)
+        return ns_sm100.UpdateJob([torch.zeros(m, n)], [torch.zeros(m, n)], [torch.zeros(m, n)], options, apart=apart)
+
+    jobs = [job(64, 64, False), job(64, 128, True), job(64, 192, True), job(64, 256, False), job(64, 320, False)]
+    events = []
+    plan = type("P", (), dict(lock=contextlib.nullcontext()))
+    monkeypatch.setattr(CH, "plan_for", lambda specs, device: plan)
+    monkeypatch.setattr(ns_sm100, "_muon_update_chain",
+                        lambda plan, part: events.append(["launch"] + [[x is j for x in jobs].index(True) for j in part]))
+    ns_sm100.muon_update_groups(jobs, lambda i, wrote: events.append(i))
+    assert events == [["launch", 0], 0, ["launch", 1], 1, ["launch", 2], 2, ["launch", 3, 4], 3, 4]
