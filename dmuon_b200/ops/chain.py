@@ -620,8 +620,10 @@ class Plan:
 
 
 # ---------------------------------------------------------------------------- plans that are kept
-#: what the work buffers of one plan may take together
-MAX_PLAN_BYTES = 6 << 30
+#: what the buffers of one plan may take together (the largest batch of a Muon step fills it to the byte for powers of
+#: two), and with what stands at the head of the work memory
+MAX_BUFFER_BYTES = 6 << 30
+MAX_PLAN_BYTES = MAX_BUFFER_BYTES + CONTROL_BYTES + 3 * _up(4 * MAX_MATRICES)
 MAX_PLANS = 256
 MAX_ARENAS = 8
 _programs: "OrderedDict[tuple, Program]" = OrderedDict()

@@ -125,6 +125,10 @@ def test_limits_of_a_plan():
     assert not CH.fits([_spec(0, 128, 128)])
     assert not CH.fits([_spec(1, 128, 128, coefs=COEFS * 20)])     # too many products
     assert not CH.fits([_spec(1, 128, 128)] * 17)
+    # the largest batch that a Muon step makes is a plan
+    from dmuon_b200.ops import ns_sm100
+    for m, n in ((4096, 4096), (4096, 14336), (14336, 4096), (1032, 1160)):
+        assert CH.possible((_spec(ns_sm100.max_batch(m, n), m, n),))
     # every tensor map is a kernel parameter: sixteen groups of the longest form that sixteen groups can have fit, more
     # operands than MAX_MAPS do not
     short = [_spec(1, 64 + 8 * i, 1024, coefs=COEFS[:1], restarts=()) for i in range(16)]
