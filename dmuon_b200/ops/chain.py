@@ -626,6 +626,8 @@ MAX_BUFFER_BYTES = 6 << 30
 MAX_PLAN_BYTES = MAX_BUFFER_BYTES + CONTROL_BYTES + 3 * _up(4 * MAX_MATRICES)
 MAX_PLANS = 256
 MAX_ARENAS = 8
+#: and those of all streams: two of the largest
+MAX_ARENA_BYTES = 2 * MAX_PLAN_BYTES + (1 << 20)
 _programs: "OrderedDict[tuple, Program]" = OrderedDict()
 _plans: "OrderedDict[tuple, Plan]" = OrderedDict()
 _arenas: "OrderedDict[tuple, Arena]" = OrderedDict()
@@ -657,7 +659,8 @@ def _arena_for(where: tuple, nbytes: int, device: torch.device) -> Arena:
         arena = None
         arena = _arenas[where] = Arena(nbytes, device)
     _arenas.move_to_end(where)
-    while len(_arenas) > MAX_ARENAS:
+    while len(_arenas) > MAX_ARENAS or (len(_arenas) > 1 and
+                                        sum(a.buf.numel() for a in _arenas.values()) > MAX_ARENA_BYTES):
         old, _ = _arenas.popitem(last=False)
         _drop(lambda k: k[1] == old)
     return arena

@@ -231,3 +231,19 @@ def test_jobs_whose_results_are_sent_have_launches_of_their_own(monkeypatch):
                         lambda plan, part: events.append(["launch"] + [[x is j for x in jobs].index(True) for j in part]))
     ns_sm100.muon_update_groups(jobs, lambda i, wrote: events.append(i))
     assert events == [["launch", 0], 0, ["launch", 1], 1, ["launch", 2], 2, ["launch", 3, 4], 3, 4]
+
+
+def test_work_memory_of_all_streams_is_bounded(streams):
+    dev, spec = torch.device("cuda", 0), [_spec(8, 4096, 4096)]          # some 2.1 GB
+    one = CH.plan_bytes(spec)
+    for s in range(1, 8):
+        streams["stream"] = s
+        plan = CH.plan_for(spec, dev)
+        assert CH._arenas[(0, s)] is plan.arena
+        assert sum(a.numel() for a in CH._arenas.values()) <= CH.MAX_ARENA_BYTES
+        assert len(CH._arenas) == min(s, CH.MAX_ARENA_BYTES // one)
+        assert {k[1] for k in CH._plans} == set(CH._arenas)
+    for s in range(20, 40):
+        streams["stream"] = s
+        CH.plan_for([_spec(1, 64, 128)], dev)
+    assert len(CH._arenas) == CH.MAX_ARENAS
