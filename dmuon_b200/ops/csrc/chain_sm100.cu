@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(const __grid_co
         const OpS& op = ops[entry_op(e)];
         if (e.w > 0) {
           if (!wait_count(done + entry_ctr(e), e.w, abort_flag)) {
-            fail_code = kStatusTimeoutPeerFlag;
+            fail_code = kStatusTimeoutChain;
             break;
           }
           fence_proxy_async_global();      // other CTAs' stores before this thread's bulk loads
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(const __grid_co
         // what other CTAs stored is read here: one lane acquires for the warp, the reads go to L2
         bool ready = true;
         if (lane == 0) ready = wait_count(done + entry_ctr(e), e.w, abort_flag);
-        if (!ready) fail_code = kStatusTimeoutPeerFlag;
+        if (!ready) fail_code = kStatusTimeoutChain;
         if (!__all_sync(0xffffffffu, ready)) break;
       }
       if (product) {
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
         const OpS& op = ops[entry_op(e)];
         if (e.w > 0) {
           if (!wait_count(done + entry_ctr(e), e.w, abort_flag)) {
-            fail_code = kStatusTimeoutPeerFlag;
+            fail_code = kStatusTimeoutChain;
             break;
           }
           fence_proxy_async_global();      // other CTAs' stores before this thread's bulk loads
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_pair_kernel(const __gr
         if (lane == 0 && e.w > 0 && tile.add_c) {
           // C was stored by other CTAs: one lane acquires for the warp, the reads go to L2
           ready = wait_count(done + entry_ctr(e), e.w, abort_flag);
-          if (!ready) fail_code = kStatusTimeoutPeerFlag;
+          if (!ready) fail_code = kStatusTimeoutChain;
         }
         ok = __all_sync(0xffffffffu, ready);
         if (!ok) break;

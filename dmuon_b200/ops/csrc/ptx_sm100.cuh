@@ -20,6 +20,7 @@ enum : int {
   kStatusTimeoutEpilogue = 3,   // epilogue waited too long for an accumulator
   kStatusTimeoutPeerFlag = 4,   // a flag another GPU or CTA should set never came
   kStatusBadArgument = 5,
+  kStatusTimeoutChain = 6,      // a tile of a product chain waited too long for the tiles it needs
 };
 
 // ~2 s at 1.9 GHz; far above any legitimate wait inside one kernel.

@@ -94,6 +94,7 @@ _STATUS_NAMES = {
     3: "epilogue waited for an accumulator",
     4: "wait on a peer / ready flag ran out (a rank did not signal in time)",
     5: "bad argument",
+    6: "a tile of a product chain waited for earlier tiles of its matrix (same GPU, no other rank involved)",
 }
 
 

@@ -87,4 +87,5 @@ def test_status_words_decode_to_kernel_timeout():
 
     assert issubclass(G.KernelTimeout, RuntimeError)
     assert "peer" in G.describe_status(4) and "did not signal" in G.describe_status(4)
+    assert "chain" in G.describe_status(6) and "no other rank" in G.describe_status(6)
     assert "TMA" in G.describe_status(1) and "unknown" in G.describe_status(99)
