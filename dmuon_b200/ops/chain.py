@@ -70,7 +70,7 @@ class _Args(ctypes.Structure):
     _fields_ = [
         ("ops", _VP), ("maps", _VP), ("tab", _VP), ("counters", _VP), ("work", _VP), ("status", _VP),
         ("n_ops", _I), ("n_maps", _I), ("total", _I), ("n_counters", _I), ("n_final", _I),
-        ("max_ctas", _I), ("bn", _I), ("wide", _I),
+        ("bn", _I), ("wide", _I),
         ("fin", _Final * MAX_GROUPS),
     ]
 

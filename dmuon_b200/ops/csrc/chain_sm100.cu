@@ -833,7 +833,7 @@ int launch_chain_pair(const DmuonChainArgs& a, cudaStream_t stream, int sms) {
   cudaError_t err = cudaFuncSetAttribute(chain_pair_kernel<WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          pair_smem_bytes<WIDE>(DMUON_CHAIN_MAX_OPS));
   if (err != cudaSuccess) return static_cast<int>(err);
-  int pairs = (a.max_ctas > 0 && a.max_ctas < sms ? a.max_ctas : sms) / 2;
+  int pairs = sms / 2;
   if (a.total < pairs) pairs = a.total;
   if (pairs < 1) pairs = 1;
   cudaLaunchConfig_t cfg = {};
@@ -860,8 +860,7 @@ int launch_chain(const DmuonChainArgs& a, cudaStream_t stream, int sms) {
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          chain_smem_bytes<BN>(DMUON_CHAIN_MAX_OPS));
   if (err != cudaSuccess) return static_cast<int>(err);
-  int grid = a.max_ctas > 0 && a.max_ctas < sms ? a.max_ctas : sms;
-  if (a.total < grid) grid = a.total;
+  const int grid = a.total < sms ? a.total : sms;
   kern<<<grid, kChainThreads, bytes, stream>>>(make_params(a));
   count_launch();
   return static_cast<int>(cudaGetLastError());

@@ -54,7 +54,7 @@ struct DmuonChainArgs {
   int* counters;               // device, zero between launches: ticket, exits, one per matrix
   void* work;                  // device: what the operations' offsets count from
   int* status;
-  int n_ops, n_maps, total, n_counters, n_final, max_ctas;
+  int n_ops, n_maps, total, n_counters, n_final;
   int bn;                      // 64 or 128: 128 x bn tiles; 256: CTA pairs on 256 x 256 tiles
   int wide;                    // CTA pairs: entries may be two tiles side by side
   struct DmuonChainFinal fin[DMUON_CHAIN_MAX_GROUPS];
