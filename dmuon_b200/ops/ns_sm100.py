@@ -256,9 +256,11 @@ def _run(ws: _Workspace, coefs, restarts, formulation: str, left: bool, xs: _XSc
 
 def _chain_pays(specs: Sequence[CH.GroupSpec]) -> bool:
     """Run these groups as one launch of the product-chain kernel?  Wherever a plan can
-    hold them: products only, one launch against one per product, B200: 105 / 231 us for
-    one matrix of 256 x 1024, 271 / 361 for 1152 x 4304, 309 / 668 for eight of
-    1024 x 1408, 1089 / 1237 for one of 3072 x 8192."""
+    hold them, because no size was found where a launch per product is faster by more than
+    calls of one form differ (4 %).  Products only, one launch against one per product, B200:
+    105 / 231 us for one matrix of 256 x 1024, 271 / 361 for 1152 x 4304, 309 / 668 for eight
+    of 1024 x 1408, 1089 / 1237 for one of 3072 x 8192; the whole call for one of
+    4096 x 14336: 2205 / 2183."""
     return CH.possible(tuple(specs))
 
 
