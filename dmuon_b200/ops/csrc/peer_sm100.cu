@@ -121,14 +121,15 @@ __global__ void wait_flags_kernel(const DmuonWaitArgs a) {
 // kW: compile-time upper bound of the number of sources (1, 2, 4 or 8).  The per-thread buffer of loads in
 // flight is kW x 8 floats, so the one-source form (a gradient already reduced in the switch) and the
 // two-rank form keep four times the occupancy of the eight-rank form.
-template <typename TG, typename TM, typename TX, int kW>
+// kAgain (second pass, see DmuonPrologueArgs::again) is compiled apart for the same reason: as a run-time switch it
+// took the two- and four-source forms from 48 and 60 registers to 56 and 66, five and four blocks an SM to four and three.
+template <typename TG, typename TM, typename TX, int kW, bool kAgain>
 __global__ void __launch_bounds__(kBlock) peer_prologue_kernel(const DmuonPeerPrologueArgs a) {
   if (a.ready_flags != nullptr) {
     if (!block_wait_flags(a.ready_flags, 0, a.world, a.ready_want, a.budget_cycles, a.status)) return;
   }
   const int t = blockIdx.y;
-  const bool again = a.again != nullptr;
-  if (again && a.again[a.slot[t]] == 0) return;
+  if (kAgain && a.again[a.slot[t]] == 0) return;
   const long long off = a.offset[t];
   TM* m = reinterpret_cast<TM*>(a.mom[t]);
   TX* x = reinterpret_cast<TX*>(a.x[t]);
@@ -171,10 +172,10 @@ __global__ void __launch_bounds__(kBlock) peer_prologue_kernel(const DmuonPeerPr
 #pragma unroll
       for (int k = 0; k < kVec; ++k) {
         const float gg = sum[k] * gs;
-        if (!again) mv[k] = Cv<TM>::to(Cv<TM>::from(fmaf(mu, mv[k], gg)));
+        if (!kAgain) mv[k] = Cv<TM>::to(Cv<TM>::from(fmaf(mu, mv[k], gg)));
         uv[k] = a.nesterov ? fmaf(mu, mv[k], gg) : mv[k];
       }
-      if (!again) st8<TM>(m + i * kVec, mv);
+      if (!kAgain) st8<TM>(m + i * kVec, mv);
     } else {
 #pragma unroll
       for (int k = 0; k < kVec; ++k) uv[k] = sum[k] * gs;
@@ -193,14 +194,14 @@ __global__ void __launch_bounds__(kBlock) peer_prologue_kernel(const DmuonPeerPr
     const float gg = s * gs;
     float u = gg;
     if (m != nullptr) {
-      const TM mn = again ? m[i] : Cv<TM>::from(fmaf(mu, Cv<TM>::to(m[i]), gg));
-      if (!again) m[i] = mn;
+      const TM mn = kAgain ? m[i] : Cv<TM>::from(fmaf(mu, Cv<TM>::to(m[i]), gg));
+      if (!kAgain) m[i] = mn;
       u = a.nesterov ? fmaf(mu, Cv<TM>::to(mn), gg) : Cv<TM>::to(mn);
     }
     x[i] = Cv<TX>::from(u * xs);
     acc = fmaf(u, u, acc);
   }
-  if (again) return;
+  if (kAgain) return;
   const float total = blk_sum(acc);
   if (threadIdx.x == 0 && a.sumsq != nullptr && !(total == 0.f)) atomicAdd(a.sumsq + a.slot[t], total);
 }
@@ -310,8 +311,15 @@ extern "C" int dmuon_peer_prologue(const DmuonPeerPrologueArgs* a, void* stream_
 #define DMUON_PEER_PROLOGUE_LAUNCH(KW)                                                                     \
   DMUON_PEER_DISPATCH(a->grad_dtype, TG,                                                                  \
     DMUON_PEER_DISPATCH(a->mom_dtype, TM,                                                                 \
-      DMUON_PEER_DISPATCH(a->x_dtype, TX, peer_prologue_kernel<TG, TM, TX, KW><<<grid, kBlock, 0, st>>>(*a))))
-  if (a->world <= 1) {
+      DMUON_PEER_DISPATCH(a->x_dtype, TX, peer_prologue_kernel<TG, TM, TX, KW, false><<<grid, kBlock, 0, st>>>(*a))))
+  if (a->again != nullptr) {
+    if (a->x_dtype != DMUON_FP16 || a->xscale == nullptr) return -1;
+    for (int i = 0; i < a->n; ++i)
+      if (a->mom[i] == nullptr) return -1;
+    DMUON_PEER_DISPATCH(a->grad_dtype, TG,
+      DMUON_PEER_DISPATCH(a->mom_dtype, TM,
+        peer_prologue_kernel<TG, TM, __half, DMUON_MAX_PEERS, true><<<grid, kBlock, 0, st>>>(*a)));
+  } else if (a->world <= 1) {
     DMUON_PEER_PROLOGUE_LAUNCH(1);
   } else if (a->world <= 2) {
     DMUON_PEER_PROLOGUE_LAUNCH(2);

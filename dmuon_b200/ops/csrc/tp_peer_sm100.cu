@@ -28,11 +28,11 @@ __device__ __forceinline__ float tp_block_sum(float v) {
   return t;
 }
 
-template <typename TG, typename TM, typename TX>
+// kAgain: second pass, see DmuonPrologueArgs::again
+template <typename TG, typename TM, typename TX, bool kAgain>
 __global__ void __launch_bounds__(kBlock) tp_gather_prologue_kernel(const DmuonTpGatherArgs a) {
   const int t = blockIdx.y;
-  const bool again = a.again != nullptr;
-  if (again && a.again[a.slot[t]] == 0) return;
+  if (kAgain && a.again[a.slot[t]] == 0) return;
   const TG* g = reinterpret_cast<const TG*>(a.src[t]);
   TM* m = reinterpret_cast<TM*>(a.mom[t]);
   TX* x = reinterpret_cast<TX*>(a.x[t]);
@@ -58,10 +58,10 @@ __global__ void __launch_bounds__(kBlock) tp_gather_prologue_kernel(const DmuonT
 #pragma unroll
         for (int k = 0; k < kVec; ++k) {
           const float gg = gv[k] * gs;
-          if (!again) mv[k] = Conv<TM>::to(Conv<TM>::from(fmaf(mu, mv[k], gg)));
+          if (!kAgain) mv[k] = Conv<TM>::to(Conv<TM>::from(fmaf(mu, mv[k], gg)));
           uv[k] = a.nesterov ? fmaf(mu, mv[k], gg) : mv[k];
         }
-        if (!again) store8<TM>(m + d, mv);
+        if (!kAgain) store8<TM>(m + d, mv);
       } else {
 #pragma unroll
         for (int k = 0; k < kVec; ++k) uv[k] = gv[k] * gs;
@@ -81,15 +81,15 @@ __global__ void __launch_bounds__(kBlock) tp_gather_prologue_kernel(const DmuonT
       const float gg = Conv<TG>::to(g[i]) * gs;
       float u = gg;
       if (m != nullptr) {
-        const TM mn = again ? m[d] : Conv<TM>::from(fmaf(mu, Conv<TM>::to(m[d]), gg));
-        if (!again) m[d] = mn;
+        const TM mn = kAgain ? m[d] : Conv<TM>::from(fmaf(mu, Conv<TM>::to(m[d]), gg));
+        if (!kAgain) m[d] = mn;
         u = a.nesterov ? fmaf(mu, Conv<TM>::to(mn), gg) : Conv<TM>::to(mn);
       }
       x[d] = Conv<TX>::from(u * xs);
       acc = fmaf(u, u, acc);
     }
   }
-  if (again) return;
+  if (kAgain) return;
   const float total = tp_block_sum(acc);
   if (threadIdx.x == 0 && a.sumsq != nullptr && !(total == 0.f)) atomicAdd(a.sumsq + a.slot[t], total);
 }
@@ -163,9 +163,17 @@ extern "C" int dmuon_tp_gather_prologue(const DmuonTpGatherArgs* a, void* stream
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream_v);
   dim3 grid(tp_grid_x((mx + kVec - 1) / kVec, a->n), a->n);
-  DMUON_TP_DISPATCH(a->src_dtype, TG,
-    DMUON_TP_DISPATCH(a->mom_dtype, TM,
-      DMUON_TP_DISPATCH(a->x_dtype, TX, tp_gather_prologue_kernel<TG, TM, TX><<<grid, kBlock, 0, st>>>(*a))));
+  if (a->again != nullptr) {
+    if (a->x_dtype != DMUON_FP16 || a->xscale == nullptr) return -1;
+    for (int i = 0; i < a->n; ++i)
+      if (a->mom[i] == nullptr) return -1;
+    DMUON_TP_DISPATCH(a->src_dtype, TG,
+      DMUON_TP_DISPATCH(a->mom_dtype, TM, tp_gather_prologue_kernel<TG, TM, __half, true><<<grid, kBlock, 0, st>>>(*a)));
+  } else {
+    DMUON_TP_DISPATCH(a->src_dtype, TG,
+      DMUON_TP_DISPATCH(a->mom_dtype, TM,
+        DMUON_TP_DISPATCH(a->x_dtype, TX, tp_gather_prologue_kernel<TG, TM, TX, false><<<grid, kBlock, 0, st>>>(*a))));
+  }
   count_launch();
   return static_cast<int>(cudaGetLastError());
 }
