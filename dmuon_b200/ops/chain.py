@@ -6,7 +6,7 @@ groups: the list of products and the tile list, on the device, used by every cal
 the same shapes.  A *plan* is a program with work memory: the buffers of one stream and
 the tensor maps over them (which travel as parameters of each launch).  A call supplies
 only what changes: where the results go and the scale of the last product (plus the
-operands, written into ``plan.X[i]`` beforehand).
+operands, written into ``plan.X[group][matrix]`` beforehand).
 
 The tile list is ordered product by product, all groups side by side; every entry
 names the number of finished warps its matrix must show before the tile may start
@@ -566,11 +566,15 @@ class Plan:
         self.program, self.arena, self.lock = program, arena, arena.lock
         self.specs, self.device, self.n_matrices, self.k = program.specs, program.device, program.n_matrices, program.k
         n = self.n_matrices
-        self.X = [arena.at(*g["X"]) for g in program.groups]
         self.sumsq = arena.control[2 + n : 2 + 2 * n].view(torch.float32)
         self.vec = arena.at(program.vec, (n,), torch.float32)
         self.vec2 = arena.at(program.vec2, (n,), torch.float32)
         self.again = arena.at(program.again, (n,), torch.int32)
+        # per group: the operands, their sums of squares and flags
+        bounds = list(zip(program.first, program.first[1:]))
+        self.X = [list(arena.at(*g["X"])) for g in program.groups]
+        self.group_sumsq = [self.sumsq[lo:hi] for lo, hi in bounds]
+        self.group_again = [self.again[lo:hi] for lo, hi in bounds]
         base = arena.buf.data_ptr()
         self._maps, maps_at = program.encode(base)
         a = _Args()

@@ -309,7 +309,7 @@ def newton_schulz_batched(
             with plan.lock:
                 plan.begin()
                 MT.clip_sumsq(mats, range(L), plan.sumsq)
-                MT.cast(mats, [X[i] for i in range(L)], slots=range(L), sumsq=plan.sumsq, norm_num=K, norm_eps=eps)
+                MT.cast(mats, X, slots=range(L), sumsq=plan.sumsq, norm_num=K, norm_eps=eps)
                 plan.run([dict(out=res)])
             if res is not out:
                 out.copy_(res)
@@ -503,11 +503,11 @@ def _muon_update_chain(plan: "CH.Plan", jobs: Sequence[UpdateJob]) -> None:
     prescales = [_prescale_of(j.moms) for j in jobs]
     plan.begin()
     passes: list = []
-    for j, X, pre, lo in zip(jobs, plan.X, prescales, plan.program.first):
-        n, o = len(j.moms), j.options
-        blocks = MT.muon_prologue(j.grads, j.moms, list(X), range(n), plan.sumsq[lo : lo + n], o["mu"], o["nesterov"],
-                                  o["gscale"], xscale=pre)
-        passes.append((blocks, plan.again[lo : lo + n]))
+    for j, X, pre, sumsq, again in zip(jobs, plan.X, prescales, plan.group_sumsq, plan.group_again):
+        o = j.options
+        blocks = MT.muon_prologue(j.grads, j.moms, X, range(len(X)), sumsq, o["mu"], o["nesterov"], o["gscale"],
+                                  xscale=pre)
+        passes.append((blocks, again))
     MT.rescale(plan.sumsq, plan.k, prescales, plan.vec, plan.vec2, plan.again, eps)
     for blocks, again in passes:
         MT.muon_prologue_again(blocks, again)
